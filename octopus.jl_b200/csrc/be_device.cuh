@@ -81,6 +81,70 @@ __device__ __noinline__ void faddeeva_upper(double zr, double zi, double &wr, do
     wi = ti + ii;
 }
 
+__device__ __forceinline__ bool faddeeva_is_far(double x, double y) {  // x, y >= 0: faddeeva_upper's own switch
+    return y > 7.0 || (x > 6.0 && (y > 0.1 || (x > 8.0 && y > 1e-10) || x > 28.0));
+}
+
+// x / d rounded as the division rounds it, from rd = 1 / d to the last bit: a multiplication and one residual step.
+__device__ __forceinline__ double div_by(double x, double d, double rd) {
+    const double q = x * rd;
+    return fma(fma(-q, d, x), rd, q);
+}
+
+// w at two first-quadrant points of the rational approximation's region: faddeeva_upper's expressions with the two
+// points' Horner chains interleaved, so that four dependent multiply-adds are in flight a thread instead of two.
+// (Goertzel's recurrence halves the polynomial's operations and gained 5 % of the soft-Gaussian collide, but it
+// rounds differently from the chains: near the axis, where the kick is a small difference of two w, its distance
+// from the same approximation in extended precision is half as large again.)
+struct WPoint {
+    double dr, zr, inv, Zr, Zi, pr, pi;
+    __device__ __forceinline__ WPoint(double zr_, double zi) : zr(zr_), pr(0.0), pi(0.0) {
+        const double L = c_weideman[0], nr = L - zi;
+        dr = L + zi;
+        inv = 1.0 / (dr * dr + zr * zr);
+        Zr = (nr * dr - zr * zr) * inv;
+        Zi = (zr * dr + nr * zr) * inv;
+    }
+    __device__ __forceinline__ void step(int k) {
+        const double tr = fma(pr, Zr, fma(-pi, Zi, c_weideman[1 + k]));
+        pi = fma(pr, Zi, pi * Zr);
+        pr = tr;
+    }
+    __device__ __forceinline__ void value(double &wr, double &wi) const {
+        constexpr double kInvSqrtPi = 0.56418958354775628695;
+        const double d2r = dr * dr - zr * zr, d2i = -(2.0 * dr * zr);
+        const double m = d2r * d2r + d2i * d2i, r0 = inv * inv;
+        const double inv2 = fma(fma(-m, r0, 1.0), r0, r0);  // 1 / m from (1 / |D|^2)^2
+        const double ar = 2.0 * pr, ai = 2.0 * pi;
+        wr = (ar * d2r + ai * d2i) * inv2 + (kInvSqrtPi * dr) * inv;
+        wi = (ai * d2r - ar * d2i) * inv2 + (kInvSqrtPi * zr) * inv;
+    }
+};
+struct WPair {
+    double r1, i1, r2, i2;
+};
+__device__ __forceinline__ WPair faddeeva_pair(double ax, double ay, double bx, double by) {
+    WPoint p(ax, ay), q(bx, by);
+#pragma unroll
+    for (int k = 0; k < kWeidemanN; ++k) {
+        p.step(k);
+        q.step(k);
+    }
+    WPair w;
+    p.value(w.r1, w.i1);
+    q.value(w.r2, w.i2);
+    return w;
+}
+// The same where a point lies in the far region.  (The rare regimes return by value: a reference to a variable of the
+// hot path would keep that variable in local memory on the hot path too.)
+__device__ __noinline__ WPair faddeeva_pair_far(double ax, double ay, double bx, double by) {
+    WPair w;
+    faddeeva_upper(ax, ay, w.r1, w.i1);
+    faddeeva_upper(bx, by, w.r2, w.i2);
+    return w;
+}
+
+constexpr double kEtaOuter = 4.412119158251195e-4;  // (8/3 * 64 * eps)^(1/4): be_eta_bounds' outer
 __device__ __forceinline__ void be_eta_bounds(double &inner, double &outer) {
     outer = sqrt(sqrt((8.0 / 3.0) * 64.0 * 2.220446049250313e-16));
     inner = outer / 2.0;
@@ -315,6 +379,101 @@ __device__ __forceinline__ void be_response(double kbb, double sigx, double sigy
                                             double &Ky, double &Hx, double &Hy) {
     if (sigx >= sigy) be_response_principal(kbb, sigx, sigy, x, y, Kx, Ky, Hx, Hy);
     else be_response_principal(kbb, sigy, sigx, y, x, Ky, Kx, Hy, Hx);
+}
+
+// The elliptic regime (eta >= outer) of the response, everything that does not depend on the point computed once:
+// be_shape per particle in the soft-Gaussian kick (the drift transports the variances), per task in the hybrid's.
+// ok = 0 outside that regime; the general response above then applies.
+struct BeShape {
+    double s1, s2;      // the long and the short axis's sigma
+    double a, d;        // their squares
+    double ia, id;      // 1 / a, 1 / d
+    double den, iden;   // sqrt(2) sqrt(a - d) and its reciprocal
+    double r, ir;       // s2 / s1, s1 / s2
+    double A;           // 2 sqrt(pi) / den
+    int swap, ok;       // swap: the long axis is y
+};
+// sqrt(v) and a reciprocal of it, v > 0
+__device__ __forceinline__ double sqrt_by(double v, double &rs) {
+    rs = rsqrt(v);
+    const double s = v * rs;
+    return fma(fma(-s, s, v), 0.5 * rs, s);
+}
+__device__ __forceinline__ BeShape be_shape(double vx, double vy) {  // the variances along x and y, positive
+    BeShape S;
+    S.swap = vx < vy;
+    double r1, r2, rt;
+    S.s1 = sqrt_by(S.swap ? vy : vx, r1);
+    S.s2 = sqrt_by(S.swap ? vx : vy, r2);
+    S.a = S.s1 * S.s1;
+    S.d = S.s2 * S.s2;
+    r1 = fma(fma(-S.s1, r1, 1.0), r1, r1);
+    r2 = fma(fma(-S.s2, r2, 1.0), r2, r2);
+    S.r = div_by(S.s2, S.s1, r1);
+    S.ir = div_by(S.s1, S.s2, r2);
+    S.ia = r1 * r1;
+    S.id = r2 * r2;
+    const double t2 = S.a - S.d;
+    S.ok = t2 >= kEtaOuter * (S.a + S.d);
+    S.den = 1.4142135623730951 * sqrt_by(t2, rt);
+    rt *= 0.70710678118654752;
+    S.iden = fma(fma(-S.den, rt, 1.0), rt, rt);
+    S.A = div_by(2.0 * 1.7724538509055159, S.den, S.iden);
+    return S;
+}
+// Kick and potential Hessians per unit kbb along x and y, and e = exp(-(x^2/varx + y^2/vary)/2).
+struct BeKick {
+    double Kx, Ky, Hx, Hy, e;
+};
+__device__ __noinline__ BeKick be_shape_axis(double s1, double s2, double x, double y) {
+    BeKick k;
+    be_axis_series(1.0, s1, s2, x, y, k.Kx, k.Hx);
+    be_axis_series(1.0, s2, s1, y, x, k.Ky, k.Hy);
+    return k;
+}
+// Outside the elliptic regime: the general response and its own exponential.
+__device__ __noinline__ BeKick be_general(double sigx, double sigy, double x, double y) {
+    BeKick k;
+    be_response(1.0, sigx, sigy, x, y, k.Kx, k.Ky, k.Hx, k.Hy);
+    k.e = exp(-0.5 * (x * x / (sigx * sigx) + y * y / (sigy * sigy)));
+    return k;
+}
+// The elliptic response.  A point takes one exponential, the two divisions of faddeeva_pair and about 420 other FP64
+// operations; the general response divides about 28 times and takes two exponentials and five square roots for the
+// same numbers.
+__device__ __forceinline__ BeKick be_shape_response(const BeShape &S, double px, double py) {
+    const double x = S.swap ? py : px, y = S.swap ? px : py;
+    const double rho2 = div_by(x * x, S.a, S.ia) + div_by(y * y, S.d, S.id);
+    BeKick k;
+    // near the axis (be_near_axis, squared and without its division and square roots): the radial series
+    const double rho4 = rho2 * rho2;
+    if (rho4 * rho2 * rho4 * rho4 * (S.a - S.d) <= 4.930380657631324e-32 * (S.a + S.d)) {
+        k = be_shape_axis(S.s1, S.s2, x, y);
+        k.e = exp(-0.5 * rho2);
+    } else {
+        const double ax = fabs(x), ay = fabs(y);
+        const double z1r = div_by(ax, S.den, S.iden), z1i = div_by(ay, S.den, S.iden);
+        const double z2r = div_by(S.r * ax, S.den, S.iden), z2i = div_by(S.ir * ay, S.den, S.iden);
+        WPair w;
+        if (faddeeva_is_far(z1r, z1i) || faddeeva_is_far(z2r, z2i)) w = faddeeva_pair_far(z1r, z1i, z2r, z2i);
+        else w = faddeeva_pair(z1r, z1i, z2r, z2i);
+        k.e = exp(-0.5 * rho2);
+        const double rr = S.A * (w.r1 - k.e * w.r2), ri = S.A * (w.i1 - k.e * w.i2);
+        k.Kx = x < 0 ? -ri : ri;
+        k.Ky = y < 0 ? -rr : rr;
+        const double t1 = x * k.Kx + y * k.Ky, it2 = 2.0 * S.iden * S.iden;
+        k.Hx = (t1 - 2.0 * (1.0 - k.e * S.r)) * it2;
+        k.Hy = (2.0 * (1.0 - k.e * S.ir) - t1) * it2;
+    }
+    if (S.swap) {
+        double t = k.Kx;
+        k.Kx = k.Ky;
+        k.Ky = t;
+        t = k.Hx;
+        k.Hx = k.Hy;
+        k.Hy = t;
+    }
+    return k;
 }
 
 // Transverse moments of a Gaussian: its centroid (unused by the kick) and the covariance entries of

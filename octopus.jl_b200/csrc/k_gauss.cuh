@@ -15,8 +15,15 @@
 
 namespace octo {
 
-constexpr int kGaussChunk = 8192;    // particles per partial-sum / kick block
+constexpr int kGaussChunk = 2048;    // particles per partial-sum block
 constexpr int kGaussThreads = 256;
+// Particles per kick block: kGaussThreads times 1 to kGaussPer, the largest that leaves kGaussWaves waves of the
+// device's kick blocks in a front (gauss_kick_chunk).  At 8192 particles a block, a front of the production beams
+// was 450 blocks on 444 slots, and half as many particles left half of the slots empty (a block's particles are
+// independent, so nothing but the density's fold order depends on the split).
+constexpr int kGaussPer = 4;
+constexpr int kGaussWaves = 4;
+constexpr int kGaussKickBlocks = 3;  // kick blocks per SM (k_gauss_kick's launch bound)
 constexpr int kGaussSums = 14;        // dx, dpx, dy, dpy, dx^2, dpx^2, dy^2, dpy^2, dx dpx, dy dpy, and the
                                       // coupled dx dy, dx dpy, dpx dy, dpx dpy
 
@@ -51,7 +58,12 @@ struct GaussArgs {
     int longitudinal;
     int drift;              // virtual drift with the longitudinal kick: 0 Hirata, 1 chromatic, 2 exact
     int coupled;            // include_sigma_xy: the full transverse covariance
+    int chunk;              // particles per kick block
 };
+inline int gauss_kick_chunk(long long front_particles, int sms) {
+    const long long per = front_particles / ((long long)kGaussThreads * kGaussWaves * kGaussKickBlocks * sms);
+    return kGaussThreads * (int)(per < 1 ? 1 : per > kGaussPer ? kGaussPer : per);
+}
 
 // The virtual drifts to and from the collision point (strong_beam.jl:517-606): forward returns S.  Without the
 // longitudinal kick the solver uses the frozen-longitudinal paraxial drift (gaussian.jl:148-150).
@@ -153,14 +165,34 @@ __global__ void __launch_bounds__(kGaussThreads) k_gauss_sums(GaussArgs A) {
     }
 }
 
-// Block b0 .. b0 + nb - 1 of k_gauss_sums belong to slice blockIdx.x (first block index in first[]).
+// Block b0 .. b0 + nb - 1 of k_gauss_sums belong to slice blockIdx.x (first block index in first[]).  16 groups of
+// threads take every 16th partial, one sum a thread, and the groups are folded in order: one thread adding a
+// production slice's partials one by one took 11 us a front.
+constexpr int kGaussFold = 16;
 template <class R>
-__global__ void k_gauss_moments(GaussArgs A, const int *first, const int *count) {
+__global__ void __launch_bounds__(16 * kGaussFold) k_gauss_moments(GaussArgs A, const int *first, const int *count) {
     pdl_wait();
     pdl_release();
-    if (threadIdx.x != 0) return;
-    const int si = blockIdx.x;
+    const int si = blockIdx.x, g = threadIdx.x >> 4, q = threadIdx.x & 15;
     const GSlice S = A.slices[si];
+    __shared__ double red[kGaussFold][16];
+    double v = 0.0;
+    if (q < kGaussSums) {
+        const double *p = A.partial + (size_t)first[si] * kGaussSums + q;
+        const int nb = count[si];
+#pragma unroll 4
+        for (int b = g; b < nb; b += kGaussFold) v += p[(size_t)b * kGaussSums];
+    }
+    red[g][q] = v;
+    __syncthreads();
+    if (g == 0) {
+#pragma unroll
+        for (int h = 1; h < kGaussFold; ++h) v += red[h][q];
+        red[0][q] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    const double *s = red[0];
     GMoments M{};
     const double floor2 = A.min_sigma * A.min_sigma;
     if (S.n == 0) {
@@ -170,10 +202,6 @@ __global__ void k_gauss_moments(GaussArgs A, const int *first, const int *count)
         A.mom[si] = M;
         return;
     }
-    double s[kGaussSums] = {};
-    for (int b = first[si]; b < first[si] + count[si]; ++b)
-#pragma unroll
-        for (int q = 0; q < kGaussSums; ++q) s[q] += A.partial[(size_t)b * kGaussSums + q];
     const double x0 = gcol<R>(A, S.beam, 0)[S.start], px0 = gcol<R>(A, S.beam, 1)[S.start],
                  y0 = gcol<R>(A, S.beam, 2)[S.start], py0 = gcol<R>(A, S.beam, 3)[S.start];
     // slicing.jl:739-770: means from the shifted sums, variances muladd(-m, m, sum2 / n), floors
@@ -208,25 +236,34 @@ __global__ void k_gauss_moments(GaussArgs A, const int *first, const int *count)
 
 // _apply_slice_kick_one! (gaussian.jl:152-185) with the uncoupled _cp_covariance_kick (strong_beam.jl:619-632)
 // between the virtual drifts above.
-// Three blocks per SM (at most 85 registers): the Bassetti-Erskine response is an FP64 latency chain, and
-// occupancy hides it better than registers do (measured: 10.6 ms per production collide at one block per
-// SM, 9.4 at two, 9.0 at three).
-template <class R>
-__global__ void __launch_bounds__(kGaussThreads, 3) k_gauss_kick(GaussArgs A) {
+// Bound by the FP64 chain of the response.  Three blocks per SM (80 registers, a few spills into L1): a turn of
+// 1.28M + 0.512M particles, 15 slices takes 2.64 ms at two blocks, 2.54 at three and 2.71 at four.  The same turn
+// took 7.47 ms with the general response in every lane (28 divisions, two exponentials, local-memory operands of its
+// calls) and 8192 particles a block.
+// COUPLED: include_sigma_xy, its own instantiation (its kick passes the coordinates by reference, which keeps them in
+// local memory).
+template <class R, bool COUPLED>
+__global__ void __launch_bounds__(kGaussThreads, kGaussKickBlocks) k_gauss_kick(const __grid_constant__ GaussArgs A) {
     pdl_wait();
     pdl_release();
+    // the task, its moments and the slice's arrays are read from shared memory where they are used: in registers they
+    // take half of a thread's 80
+    __shared__ GTask T;
+    __shared__ GMoments M;
+    __shared__ R *c[6];
     const int2 bm = A.blockmap[blockIdx.x];
-    const GTask T = A.tasks[bm.x];
-    const GMoments M = A.mom[T.mom];
-    R *c[6];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) c[q] = gcol<R>(A, T.fld_beam, q);
+    if (threadIdx.x == 0) {
+        T = A.tasks[bm.x];
+        M = A.mom[T.mom];
+        for (int q = 0; q < 6; ++q) c[q] = gcol<R>(A, T.fld_beam, q) + T.fld_start;
+    }
+    __syncthreads();
     const bool lk = A.longitudinal != 0;
     const double twopi = 6.283185307179586476925286766559005768394338;
     double dens = 0.0;
-    const long long end = min(T.fld_n, (long long)bm.y + kGaussChunk);
-    for (long long k = bm.y + threadIdx.x; k < end; k += kGaussThreads) {
-        const long long i = T.fld_start + k;
+    const int end = (int)min((long long)A.chunk, T.fld_n - bm.y);
+    for (int k = threadIdx.x; k < end; k += kGaussThreads) {
+        const int i = bm.y + k;
         double x = c[0][i], px = c[1][i], y = c[2][i], py = c[3][i], z = c[4][i], pz = c[5][i];
         const double S = drift_forward(A.drift, lk, x, px, y, py, z, pz, T.center);
         const double xx = x - M.mx + M.mpx * S;
@@ -237,17 +274,17 @@ __global__ void __launch_bounds__(kGaussThreads, 3) k_gauss_kick(GaussArgs A) {
         const double d = M.d0 - 2 * S * M.bypy + S * S * M.qyy;
         const double au = 2 * (M.bxx - S * M.qxx);
         const double du = 2 * (M.bypy - S * M.qyy);
-        double density = 0.0;
-        if (A.coupled) coupled_kick(M, T.kbb, S, xx, yy, px, py, pz, density);
-        else if (!(a <= 0 || d <= 0)) {
-            const double sigx = sqrt(a), sigy = sqrt(d);
-            double Kx, Ky, Hxx, Hyy;
-            be_response(T.kbb, sigx, sigy, xx, yy, Kx, Ky, Hxx, Hyy);
-            const double expterm = exp(-0.5 * (xx * xx / (sigx * sigx) + yy * yy / (sigy * sigy)));
-            px += Kx * T.kbb;
-            py += Ky * T.kbb;
-            pz += 0.25 * (Hxx * au + Hyy * du);
-            density = expterm / twopi / sigx / sigy;
+        double density = 0.0;  // times 2 pi
+        if (COUPLED) {
+            coupled_kick(M, T.kbb, S, xx, yy, px, py, pz, density);
+            density *= twopi;
+        } else if (!(a <= 0 || d <= 0)) {
+            const BeShape B = be_shape(a, d);
+            const BeKick K = B.ok ? be_shape_response(B, xx, yy) : be_general(sqrt(a), sqrt(d), xx, yy);
+            px += K.Kx * T.kbb;
+            py += K.Ky * T.kbb;
+            pz += 0.25 * (T.kbb * K.Hx * au + T.kbb * K.Hy * du);
+            density = K.e * B.ir * B.ia;  // 1 / (sigma_x sigma_y) = (s1 / s2) / s1^2
         }
         if (lk) pz += 0.5 * ((px - px0) * M.mpx + (py - py0) * M.mpy);
         else pz = pz0;
@@ -258,7 +295,7 @@ __global__ void __launch_bounds__(kGaussThreads, 3) k_gauss_kick(GaussArgs A) {
         c[3][i] = (R)py;
         c[4][i] = (R)z;
         c[5][i] = (R)pz;
-        dens += density * twopi;
+        dens += density;
     }
     if (!T.lum) return;
     __shared__ double red[kGaussThreads / 32];
@@ -275,16 +312,21 @@ __global__ void __launch_bounds__(kGaussThreads, 3) k_gauss_kick(GaussArgs A) {
     }
 }
 
-// Pair luminosity (gaussian.jl:64-108): sum of density * 2 pi over the sampled slice / 2 pi * klum.
-// One thread per sampling task; its kick blocks' partials in block order.
-__global__ void k_gauss_lum(GaussArgs A, const int *lum_task, const int *first, const int *count, int nlum) {
+// Pair luminosity (gaussian.jl:64-108): sum of density * 2 pi over the sampled slice / 2 pi * klum.  One warp per
+// sampling task: each lane takes every 32nd of its kick blocks' partials, then the lanes are folded pairwise.
+__global__ void __launch_bounds__(32) k_gauss_lum(GaussArgs A, const int *lum_task, const int *first, const int *count) {
     pdl_wait();
     pdl_release();
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nlum) return;
-    const GTask T = A.tasks[lum_task[k]];
+    const int k = blockIdx.x, lane = threadIdx.x;
+    const double *p = A.lum_partial + first[k];
+    const int nb = count[k];
     double s = 0.0;
-    for (int b = first[k]; b < first[k] + count[k]; ++b) s += A.lum_partial[b];
+#pragma unroll 4
+    for (int b = lane; b < nb; b += 32) s += p[b];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane) return;
+    const GTask T = A.tasks[lum_task[k]];
     const double twopi = 6.283185307179586476925286766559005768394338;
     A.lum_parts[T.pair] = s / twopi * T.klum;
 }

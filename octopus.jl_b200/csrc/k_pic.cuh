@@ -2042,6 +2042,7 @@ struct KickJob {
     int fld_beam, ok;
     int hyb;               // Gaussian-subtracted hybrid active for this task
     HybridTask H;
+    BeShape B[2];          // hyb == 1: the reference Gaussians of both boundaries
     int next_pair, next_task;  // luminosity box of the field slice's next pair (:node), or -1
     R next_sM;
 };
@@ -2222,19 +2223,22 @@ __device__ __forceinline__ void kick_particle(const Collide &C, const KickJob<R>
             // times the Bassetti-Erskine kick at both boundaries, blended in z, and its longitudinal terms.
             const HybridTask &H = J.H;
             const double kbb_eff = (double)ks * H.half_ns;
-            double bLx, bLy, HxL = 0, HyL = 0, bRx, bRy, HxR = 0, HyR = 0;
-            be_response(lk ? kbb_eff : 0.0, H.sigx[0], H.sigy[0], (double)x - H.mux[0], (double)y - H.muy[0], bLx, bLy,
-                        HxL, HyL);
-            be_response(lk ? kbb_eff : 0.0, H.sigx[1], H.sigy[1], (double)x - H.mux[1], (double)y - H.muy[1], bRx, bRy,
-                        HxR, HyR);
-            const double Kxa = H.half_ns * ((double)zL * bLx + (double)zR * bRx);
-            const double Kya = H.half_ns * ((double)zL * bLy + (double)zR * bRy);
+            BeKick L, Rr;
+            if (J.B[0].ok && J.B[1].ok) {
+                L = be_shape_response(J.B[0], (double)x - H.mux[0], (double)y - H.muy[0]);
+                Rr = be_shape_response(J.B[1], (double)x - H.mux[1], (double)y - H.muy[1]);
+            } else {
+                L = be_general(H.sigx[0], H.sigy[0], (double)x - H.mux[0], (double)y - H.muy[0]);
+                Rr = be_general(H.sigx[1], H.sigy[1], (double)x - H.mux[1], (double)y - H.muy[1]);
+            }
+            const double Kxa = H.half_ns * ((double)zL * L.Kx + (double)zR * Rr.Kx);
+            const double Kya = H.half_ns * ((double)zL * L.Ky + (double)zR * Rr.Ky);
             const double dpxa = (double)ks * Kxa, dpya = (double)ks * Kya;
             px += (R)((double)ks * (double)Kx + dpxa);
             py += (R)((double)ks * (double)Ky + dpya);
             if (lk) {
-                const double covL = (HxL * H.rx[0] + HyL * H.ry[0]) / 4.0;
-                const double covR = (HxR * H.rx[1] + HyR * H.ry[1]) / 4.0;
+                const double covL = 0.25 * kbb_eff * (L.Hx * H.rx[0] + L.Hy * H.ry[0]);
+                const double covR = 0.25 * kbb_eff * (Rr.Hx * H.rx[1] + Rr.Hy * H.ry[1]);
                 if (kPrecision) {  // summed in FP64, one rounding into the pz increment
                     dpz += (R)((double)ks * (double)Kz * (double)J.hzi + ((double)zL * covL + (double)zR * covR) +
                                0.5 * (dpxa * H.mpx + dpya * H.mpy));
@@ -2291,6 +2295,8 @@ __global__ void __launch_bounds__(kKickThreads, sizeof(R) == 8 ? 2 : 4)
         if (C.o.gaussian && J.ok) {
             J.H = C.hyb[bm.x];
             J.hyb = J.H.mode;
+            if (J.hyb == 1)
+                for (int k = 0; k < 2; ++k) J.B[k] = be_shape(J.H.sigx[k] * J.H.sigx[k], J.H.sigy[k] * J.H.sigy[k]);
         }
         J.gL = grid_r<R>(gL);
         J.gR = grid_r<R>(gR);

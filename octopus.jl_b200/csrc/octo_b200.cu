@@ -1714,11 +1714,14 @@ void CollideJob::run_gaussian(const SliceInfo &S1, const SliceInfo &S2) {
     std::vector<int2> smap, kmap;             // sums blocks, kick blocks
     std::vector<int> sfirst, scount;          // per slice: its sums blocks
     std::vector<int> ltask, lfirst, lcount;   // per sampling task: its kick blocks
-    struct Front { int s0, ns, sb0, nsb, t0, nt, kb0, nkb, l0, nl; };
+    struct Front { int s0, ns, sb0, nsb, t0, nt, kb0, nkb, l0, nl, chunk; };
     std::vector<Front> fronts;
     tasks.clear();
     for (size_t f = 0; f < batches.size(); ++f) {
-        Front F{(int)gs.size(), 0, (int)smap.size(), 0, (int)gt.size(), 0, (int)kmap.size(), 0, (int)ltask.size(), 0};
+        Front F{(int)gs.size(), 0, (int)smap.size(), 0, (int)gt.size(), 0, (int)kmap.size(), 0, (int)ltask.size(), 0, 0};
+        long long front_n = 0;
+        for (const OrderEntry &pr : batches[f]) front_n += S1.count[pr.i - 1] + S2.count[pr.j - 1];
+        F.chunk = gauss_kick_chunk(front_n, c->num_sms);
         for (const OrderEntry &pr : batches[f]) {
             const int i = pr.i, j = pr.j, p = pos_of[(size_t)(i - 1) * ns2 + (j - 1)];
             const int t0 = (int)gt.size();
@@ -1752,7 +1755,7 @@ void CollideJob::run_gaussian(const SliceInfo &S1, const SliceInfo &S2) {
                     ltask.push_back(tid);
                     lfirst.push_back((int)kmap.size());
                 }
-                for (long long off = 0; off < T.fld_n; off += kGaussChunk) kmap.push_back(make_int2(tid, (int)off));
+                for (long long off = 0; off < T.fld_n; off += F.chunk) kmap.push_back(make_int2(tid, (int)off));
                 if (T.lum) lcount.push_back((int)kmap.size() - lfirst.back());
                 gt.push_back(T);
                 Task PT{};  // for error reports
@@ -1830,7 +1833,7 @@ void CollideJob::run_gaussian(const SliceInfo &S1, const SliceInfo &S2) {
             Am.slices = c->g_slices.p + F.s0;
             Am.mom = c->g_mom.p + F.s0;
             with_real(fp32, [&](auto r) {
-                launch_pdl(k_gauss_moments<decltype(r)>, F.ns, 32, 0, st, Am, d_sfirst + F.s0, d_scount + F.s0);
+                launch_pdl(k_gauss_moments<decltype(r)>, F.ns, 16 * kGaussFold, 0, st, Am, d_sfirst + F.s0, d_scount + F.s0);
             });
             launches += (F.nsb ? 1 : 0) + 1;
         }
@@ -1839,12 +1842,13 @@ void CollideJob::run_gaussian(const SliceInfo &S1, const SliceInfo &S2) {
             GaussArgs Ak = A;
             Ak.blockmap = c->g_bmap.p + smap.size() + F.kb0;
             Ak.lum_partial = c->g_lum_partial.p + F.kb0;
+            Ak.chunk = F.chunk;
             with_real(fp32, [&](auto r) {
-                if (F.nkb) launch_pdl(k_gauss_kick<decltype(r)>, F.nkb, kGaussThreads, 0, st, Ak);
+                if (F.nkb && A.coupled) launch_pdl(k_gauss_kick<decltype(r), true>, F.nkb, kGaussThreads, 0, st, Ak);
+                else if (F.nkb) launch_pdl(k_gauss_kick<decltype(r), false>, F.nkb, kGaussThreads, 0, st, Ak);
             });
             // the fold reads the kick partials by their index over all fronts (lfirst)
-            if (F.nl) launch_pdl(k_gauss_lum, (F.nl + 31) / 32, 32, 0, st, A, d_ltask + F.l0, d_lfirst + F.l0,
-                                 d_lcount + F.l0, F.nl);
+            if (F.nl) launch_pdl(k_gauss_lum, F.nl, 32, 0, st, A, d_ltask + F.l0, d_lfirst + F.l0, d_lcount + F.l0);
             launches += (F.nkb ? 1 : 0) + (F.nl ? 1 : 0);
         }
     }

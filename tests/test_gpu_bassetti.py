@@ -1,0 +1,53 @@
+"""The Bassetti-Erskine response of the soft-Gaussian kick where its evaluation changes: the round closed form, the
+near-round series, the blend, the elliptic form just above it and at strong aspect ratios with either axis the long
+one; each at points on the axes, inside and outside the radial series' region, in the rational approximation's region
+and in the far region of w(z).  One pair of single slices, kbb = 1, so a probe's momentum is the kick itself."""
+import numpy as np
+import pytest
+
+from helpers import oracle_params, E_PARAMS, P_PARAMS
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def _source(n, sx, sy):
+    rng = np.random.default_rng(5)
+    u = rng.standard_normal(n)
+    u = (u - u.mean()) / u.std()
+    c = np.zeros((6, n))
+    c[0], c[2] = sx * u, sy * u[rng.permutation(n)]  # the same values: the sample's sigma ratio is sx / sy
+    return c
+
+
+def _probes(sx, sy, n):
+    a = np.array([0.0, 1e-3, 5e-3, 7e-3, 2e-2, 0.3, 1.0, 3.0, 6.5, 15.0, 60.0])
+    a = np.concatenate([a, -a[1:]])
+    gx, gy = np.meshgrid(a, a)
+    c = np.zeros((6, n))
+    c[0], c[2] = sx * np.resize(gx.ravel(), n), sy * np.resize(gy.ravel(), n)
+    return c
+
+
+@pytest.mark.parametrize("aspect", [1.0, 1.0 + 1e-4, 1.0 + 3e-4, 1.0 + 5e-4, 1.02, 11.0, 1.0 / 11.0, 150.0])
+@pytest.mark.parametrize("n", [441, 3 * 444 * 256 + 77])  # one particle a thread; several, with a ragged last block
+def test_kick_of_every_regime(aspect, n):
+    import octo_b200 as ob
+    sy = 1e-5
+    e, p = _source(4001, aspect * sy, sy), _probes(aspect * sy, sy, n)
+    solver = ob.GaussianPoissonSolver(slicing=ob.LongitudinalSlicing(nslices=1, method="normal_quantile"), kbb1=1.0,
+                                      kbb2=1.0, luminosity_scale=1.0, gaussian_when_luminosity=1)
+    params = [ob.BeamParams(q["charge"], q["mass"], q["energy"], q["r0"], q["npart"]) for q in (E_PARAMS, P_PARAMS)]
+    be, bp = ob.Beam.from_numpy(e, params[0]), ob.Beam.from_numpy(p, params[1])
+    lum = ob.collide(solver, be, bp)
+    opt = orc.OracleOptions(nslices1=1, nslices2=1, kbb1=1.0, kbb2=1.0, luminosity_scale=1.0)
+    ref = orc.gaussian_collide(opt, e, p, *oracle_params(), 0.0, 1, False, False, "hirata", False)
+    got = bp.numpy()
+    assert abs(lum / ref - 1.0) < 1e-12
+    # each side rounds w(z) to about 4 x 1.1e-16, and the elliptic form multiplies the difference of two such values by
+    # 2 sqrt(pi) / (sqrt(2) sqrt(2 eta) sigma) <= 84 / sigma (eta >= 4.4e-4), where the largest kick is 0.45 / sigma:
+    # 2 x 4.4e-16 x 84 / 0.45 = 1.6e-13 of it; the bound is twice that
+    for k in (1, 3):
+        assert np.max(np.abs(got[k] - p[k])) <= 3e-13 * np.max(np.abs(p[[1, 3]]))
+    # the longitudinal kick here is the drift term of the kicked momenta alone
+    assert np.max(np.abs(got[5] - p[5])) <= 2e-12 * np.max(np.abs(p[5])) + 1e-16
