@@ -3,22 +3,30 @@
 // power rows, over the live particles (all six coordinates finite) when lost particles are masked, else
 // over all particles (one non-finite particle then makes the row NaN).
 //
-// Two passes over the beam, as the definition needs the means first: k_moment_sums (six sums and the live
-// count), then k_moment_pairs (all 21 second-order sums from one read of each particle) and, for rows of
-// order 3 and more, k_moment_general in chunks.  Each writes per-block partials (a fixed block count)
-// that a fold block sums in a fixed order, so a row is deterministic for a given beam size; the folds write
-// the row into device memory, so observing a turn never synchronises the host.
+// One pass over the beam: k_moment_pass sums the six deviations from a pivot near the beam's centre and their 21
+// products, and k_moment_finish turns them into the means and the second central moments, m_ij = S_ij / n - d_i d_j
+// with d = S / n the mean's offset from the pivot.  The definition takes the means first, in a pass of its own; one
+// read of the beam instead of two, and three launches instead of six, took the rows of a 2.56M and a 1.024M-particle
+// float64 beam from 128 to 65 us of kernel time together (26 us of reading at the measured copy bandwidth).  The pivot (k_moment_pivot) is zero for
+// a centred coordinate, where d is the mean itself, and else the mean of 4096 particles spread over the beam, about
+// sigma / 64 from the mean and at most sqrt(n) / 4096 of the sigma that a stray particle makes; either way the
+// subtraction loses nothing.  (Zero matters: a mean far smaller than sigma would be the sum of a pivot and its
+// opposite, which costs it three digits.)  Rows of order 3 and more (k_moment_general) read the beam
+// again, in chunks, with the means known.  Each pass writes per-block partials (a fixed block count) that are summed
+// in a fixed order, so a row is deterministic for a given beam size; the row goes to device memory, so observing a
+// turn never synchronises the host.
 #pragma once
 #include "octo_internal.cuh"
 
 namespace octo {
 
-constexpr int kMomentBlocks = 1184;     // partial-sum blocks (a fixed count: fold order independent of the GPU)
+constexpr int kMomentBlocks = 592;      // partial-sum blocks (a fixed count: fold order independent of the GPU)
 constexpr int kMomentThreads = 256;
 constexpr int kMomentWarps = kMomentThreads / 32;
 constexpr int kMomentChunk = 8;         // rows of order >= 3 per generic pass (accumulators held in registers)
 constexpr int kMomentPairs = 21;        // second-order rows: the products of deviations (i <= j)
 constexpr int kMomentsMax = 256;
+constexpr int kMomentSums1 = 6 + kMomentPairs + 1;  // k_moment_pass: deviations, their products, the live count
 
 // Rows of order >= 3 of one generic pass.
 struct MomentPowers {
@@ -74,24 +82,116 @@ __device__ __forceinline__ void load6(double (&c)[6], const R *x, const R *px, c
     c[5] = (double)pz[i];
 }
 
+// The beam's arrays of one moment pass.
 template <class R>
-__global__ void __launch_bounds__(kMomentThreads) k_moment_sums(const R *__restrict__ x, const R *__restrict__ px,
-                                                                  const R *__restrict__ y, const R *__restrict__ py,
-                                                                  const R *__restrict__ z, const R *__restrict__ pz,
-                                                                  long long n, int mask, double *partial) {
+struct MomentBeam {
+    const R *c[6];
+    long long n;
+    int mask;
+};
+
+// Block d: coordinate d's pivot from its finite values among 4096 particles spread over the beam: their mean, or zero
+// when there is none or the mean lies within an eighth of their rms spread.
+constexpr int kPivotThreads = 1024, kPivotPer = 4;
+template <class R>
+__global__ void __launch_bounds__(kPivotThreads) k_moment_pivot(const __grid_constant__ MomentBeam<R> B, double *pivot) {
     pdl_wait();
     pdl_release();
-    __shared__ double red[7 * kMomentWarps];
-    double s[7] = {0, 0, 0, 0, 0, 0, 0};
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        double c[6];
-        load6(c, x, px, y, py, z, pz, i);
-        if (mask && !live6(c)) continue;
+    __shared__ double red[3][kPivotThreads / 32];
+    const R *c = B.c[blockIdx.x];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double v[kPivotPer], s[3] = {0.0, 0.0, 0.0};  // sum, sum of squares, count
 #pragma unroll
-        for (int d = 0; d < 6; ++d) s[d] += c[d];
-        s[6] += 1.0;
+    for (int k = 0; k < kPivotPer; ++k) {
+        const long long q = (long long)k * kPivotThreads + threadIdx.x, samples = kPivotThreads * kPivotPer;
+        // every particle of a small beam once, else 4096 of them (q n / 4096 without the product's overflow)
+        const long long i = B.n <= samples ? q : B.n / samples * q + B.n % samples * q / samples;
+        v[k] = i < B.n ? (double)c[i] : (double)NAN;
     }
-    block_sums<7>(s, red, partial);
+#pragma unroll
+    for (int k = 0; k < kPivotPer; ++k)
+        if (isfinite(v[k])) {
+            s[0] += v[k];
+            s[1] = fma(v[k], v[k], s[1]);
+            s[2] += 1.0;
+        }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+        if (lane == 0) red[k][warp] = s[k];
+    }
+    __syncthreads();
+    if (warp) return;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        s[k] = red[k][lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+    }
+    const double mean = s[0] / s[2];
+    const bool centred = 65.0 * mean * mean <= s[1] / s[2];  // mean^2 <= (mean square - mean^2) / 64
+    if (lane == 0) pivot[blockIdx.x] = isfinite(mean) && !centred ? mean : 0.0;
+}
+
+// Bound by HBM with 56 of its registers holding sums: two blocks per SM, and the next two particles' twelve loads
+// issued before the current two are summed.  Two particles' terms are added to each other before they go to the sum:
+// half as many roundings of the running sums, which is what a covariance near zero shows.
+template <class R>
+__global__ void __launch_bounds__(kMomentThreads, 2) k_moment_pass(const __grid_constant__ MomentBeam<R> B,
+                                                                   const double *pivots, double *partial) {
+    pdl_wait();
+    pdl_release();
+    __shared__ double red[kMomentSums1 * kMomentWarps];
+    double pivot[6];
+#pragma unroll
+    for (int d = 0; d < 6; ++d) pivot[d] = pivots[d];
+    double s[kMomentSums1];
+#pragma unroll
+    for (int k = 0; k < kMomentSums1; ++k) s[k] = 0.0;
+    int live = 0;
+    auto deviations = [&](const R (&v)[6], bool there, double (&dv)[6]) {
+        double c[6];
+#pragma unroll
+        for (int d = 0; d < 6; ++d) c[d] = (double)v[d];
+        const bool on = there && (!B.mask || live6(c));
+        live += on;
+#pragma unroll
+        for (int d = 0; d < 6; ++d) dv[d] = on ? c[d] - pivot[d] : 0.0;
+    };
+    auto load = [&](R (&v)[6], long long i) {
+#pragma unroll
+        for (int d = 0; d < 6; ++d) v[d] = B.c[d][i];
+    };
+    const long long step = (long long)gridDim.x * blockDim.x;
+    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    R na[6], nb[6] = {};
+    if (i < B.n) load(na, i);
+    if (i + step < B.n) load(nb, i + step);
+    while (i < B.n) {
+        R a[6], b[6];
+#pragma unroll
+        for (int d = 0; d < 6; ++d) {
+            a[d] = na[d];
+            b[d] = nb[d];
+        }
+        const bool two = i + step < B.n;
+        i += 2 * step;
+        if (i < B.n) load(na, i);
+        if (i + step < B.n) load(nb, i + step);
+        double da[6], db[6];
+        deviations(a, true, da);
+        deviations(b, two, db);
+#pragma unroll
+        for (int d = 0; d < 6; ++d) s[d] += da[d] + db[d];
+        int k = 6;
+#pragma unroll
+        for (int p = 0; p < 6; ++p)
+#pragma unroll
+            for (int q = p; q < 6; ++q, ++k) s[k] += fma(da[p], da[q], db[p] * db[q]);
+    }
+    s[kMomentSums1 - 1] = (double)live;
+    block_sums<kMomentSums1>(s, red, partial);
 }
 
 // Fixed-order sum of partial[b * stride + k] over b < nb by one block of kMomentThreads threads: thread t
@@ -110,50 +210,57 @@ __device__ __forceinline__ double fold_partials(const double *partial, int nb, i
     return s;
 }
 
-// The live count means[6] and means[0..5]; block k folds partial column k (7 blocks).
-__global__ void __launch_bounds__(kMomentThreads) k_moment_means(const double *partial, int nb, double *sums) {
+// Block d < 6: the mean of coordinate d (0 / 0 = NaN for a beam without live particles, as the reference reports it),
+// block 0 also the live count means[6] and the row's turn; block 6 + k: requested pair k, NaN where a mean it
+// involves is not finite, as the deviations from such a mean are.  The four columns a pair takes are folded together.
+__global__ void __launch_bounds__(kMomentThreads) k_moment_finish(const double *pivots, const double *partial, int nb,
+                                                                  double turn, const __grid_constant__ MomentHead head,
+                                                                  const __grid_constant__ MomentPairRows Q,
+                                                                  double *means, double *row) {
     pdl_wait();
     pdl_release();
-    const double s = fold_partials(partial, nb, 7, blockIdx.x);
-    if (threadIdx.x == 0) sums[blockIdx.x] = s;
-}
-__global__ void k_moment_divide(double *means) {
-    pdl_wait();
-    pdl_release();
-    if (threadIdx.x < 6) means[8 + threadIdx.x] = means[threadIdx.x] / means[6];
-}
-
-// All 21 second-order sums: (c_i - <c_i>) (c_j - <c_j>) for i < j, (c_i - <c_i>)^2 for i = j (the reference's
-// term 1.0 * d_i * d_j, and d_i^2 = d_i * d_i).
-template <class R>
-__global__ void __launch_bounds__(kMomentThreads) k_moment_pairs(const R *__restrict__ x, const R *__restrict__ px,
-                                                                   const R *__restrict__ y, const R *__restrict__ py,
-                                                                   const R *__restrict__ z, const R *__restrict__ pz,
-                                                                   long long n, int mask, const double *means,
-                                                                   double *partial) {
-    pdl_wait();
-    pdl_release();
-    __shared__ double red[kMomentPairs * kMomentWarps];
-    double mu[6];
-#pragma unroll
-    for (int d = 0; d < 6; ++d) mu[d] = means[8 + d];
-    double acc[kMomentPairs];
-#pragma unroll
-    for (int k = 0; k < kMomentPairs; ++k) acc[k] = 0.0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        double c[6];
-        load6(c, x, px, y, py, z, pz, i);
-        if (mask && !live6(c)) continue;
-        double dv[6];
-#pragma unroll
-        for (int d = 0; d < 6; ++d) dv[d] = c[d] - mu[d];
-        int k = 0;
-#pragma unroll
-        for (int a = 0; a < 6; ++a)
-#pragma unroll
-            for (int b = a; b < 6; ++b) acc[k++] += dv[a] * dv[b];
+    __shared__ double red[4][kMomentWarps];
+    const int q = (int)blockIdx.x - 6;
+    int a = blockIdx.x, b = blockIdx.x, pair = 0;
+    if (q >= 0) {
+        pair = Q.pair[q];
+        a = 0;
+        int first = 0;
+        while (pair >= first + 6 - a) first += 6 - a++;
+        b = a + pair - first;
     }
-    block_sums<kMomentPairs>(acc, red, partial);
+    const int col[4] = {kMomentSums1 - 1, a, b, 6 + pair};
+    double t[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int p = threadIdx.x; p < nb; p += kMomentThreads)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) t[k] += partial[(size_t)p * kMomentSums1 + col[k]];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
+        if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = t[k];
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        t[k] = 0.0;
+#pragma unroll
+        for (int w = 0; w < kMomentWarps; ++w) t[k] += red[k][w];
+    }
+    const double n = t[0], da = t[1] / n, db = t[2] / n;
+    if (q >= 0) {
+        row[1 + Q.slot[q]] = isfinite(da) && isfinite(db) ? fma(-da, db, t[3] / n) : (double)NAN;
+        return;
+    }
+    const double mean = pivots[a] + da;
+    means[8 + a] = mean;
+    for (int k = 0; k < head.n; ++k)
+        if (head.coord[k] == a) row[1 + head.slot[k]] = mean;
+    if (a == 0) {
+        means[6] = n;
+        row[0] = turn;
+    }
 }
 
 __device__ __noinline__ double ipow(double v, int p) {
@@ -203,15 +310,6 @@ __global__ void __launch_bounds__(kMomentThreads, 2) k_moment_general(const R *_
 
 // Folds of the block partials (fixed order), divided by the live count (0 / 0 = NaN for a beam without
 // live particles, as the reference reports it).  Block k folds requested row k.
-__global__ void __launch_bounds__(kMomentThreads) k_moment_fold_pairs(const double *partial, int nb,
-                                                                        const double *means, MomentPairRows Q,
-                                                                        double *row) {
-    pdl_wait();
-    pdl_release();
-    const int k = blockIdx.x;
-    const double s = fold_partials(partial, nb, kMomentPairs, Q.pair[k]);
-    if (threadIdx.x == 0) row[1 + Q.slot[k]] = s / means[6];
-}
 __global__ void __launch_bounds__(kMomentThreads) k_moment_fold(const double *partial, int nb, const double *means,
                                                                   MomentPowers P, double *row) {
     pdl_wait();
@@ -219,15 +317,6 @@ __global__ void __launch_bounds__(kMomentThreads) k_moment_fold(const double *pa
     const int k = blockIdx.x;
     const double s = fold_partials(partial, nb, kMomentChunk, k);
     if (threadIdx.x == 0) row[1 + P.slot[k]] = s / means[6];
-}
-
-// row[0] = turn and the order-1 entries (the means; NaN for a beam without live particles).
-__global__ void k_moment_row_head(const double *means, double turn, MomentHead head, double *row) {
-    pdl_wait();
-    pdl_release();
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    row[0] = turn;
-    for (int k = 0; k < head.n; ++k) row[1 + head.slot[k]] = means[8 + head.coord[k]];
 }
 
 }  // namespace octo

@@ -2773,26 +2773,22 @@ int32_t octo_beam_moments(octo_ctx *c, const octo_beam *beam, const int32_t *pow
     cudaStream_t st = (cudaStream_t)stream;
     try {
         CK(cudaSetDevice(c->device));
-        c->mom_partial.ensure((size_t)kMomentBlocks * kMomentPairs);
-        c->mom_means.ensure(16);
+        c->mom_partial.ensure((size_t)kMomentBlocks * kMomentSums1);
+        c->mom_means.ensure(24);
         const long long n = beam->n;
         const int mask = mask_lost != 0;
         with_real(beam->dtype == 1, [&](auto r) {
             using R = decltype(r);
             R *b[6] = {(R *)beam->x, (R *)beam->px, (R *)beam->y, (R *)beam->py, (R *)beam->z, (R *)beam->pz};
             const double *means = c->mom_means.p;
-            launch_pdl(k_moment_sums<R>, kMomentBlocks, kMomentThreads, 0, st, b[0], b[1], b[2], b[3], b[4], b[5], n,
-                       mask, c->mom_partial.p);
-            launch_pdl(k_moment_means, 7, kMomentThreads, 0, st, (const double *)c->mom_partial.p, (int)kMomentBlocks,
-                       c->mom_means.p);
-            launch_pdl(k_moment_divide, 1, 32, 0, st, c->mom_means.p);
-            launch_pdl(k_moment_row_head, 1, 32, 0, st, means, (double)turn, head, row);
-            if (pairs.n) {
-                launch_pdl(k_moment_pairs<R>, kMomentBlocks, kMomentThreads, 0, st, b[0], b[1], b[2], b[3], b[4],
-                           b[5], n, mask, means, c->mom_partial.p);
-                launch_pdl(k_moment_fold_pairs, pairs.n, kMomentThreads, 0, st, (const double *)c->mom_partial.p,
-                           (int)kMomentBlocks, means, pairs, row);
-            }
+            const MomentBeam<R> mb{{b[0], b[1], b[2], b[3], b[4], b[5]}, n, mask};
+            double *pivots = c->mom_means.p + 16;
+            launch_pdl(k_moment_pivot<R>, 6, kPivotThreads, 0, st, mb, pivots);
+            launch_pdl(k_moment_pass<R>, kMomentBlocks, kMomentThreads, 0, st, mb, (const double *)pivots,
+                       c->mom_partial.p);
+            launch_pdl(k_moment_finish, 6 + pairs.n, kMomentThreads, 0, st, (const double *)pivots,
+                       (const double *)c->mom_partial.p, (int)kMomentBlocks, (double)turn, head, pairs, c->mom_means.p,
+                       row);
             for (size_t g0 = 0; g0 < general.size(); g0 += kMomentChunk) {
                 MomentPowers P{};
                 P.n = (int)std::min<size_t>(kMomentChunk, general.size() - g0);
