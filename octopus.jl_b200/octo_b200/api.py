@@ -292,6 +292,9 @@ def _scratch_ctx(device: int):
     return _scratch[device].ptr
 
 
+_Mat36 = C.c_double * 36
+
+
 class Linear6D:
     """Linear 6D one-turn map (linear6d.jl:85-123, 233-280) for an uncoupled lattice without dispersion:
     per-plane rotation by 2*pi*tune with equal Twiss parameters at both ends."""
@@ -311,7 +314,7 @@ class Linear6D:
 
     def track(self, beam: Beam, turns: int = 1, stream=None):
         b = beam.to_c()
-        m = (C.c_double * 36)(*self.matrix.tolist())
+        m = _Mat36.from_buffer(np.array(self.matrix, dtype=np.float64).reshape(36))
         st = (stream or torch.cuda.current_stream(beam.coords.device)).cuda_stream
         ctx = _scratch_ctx(beam.coords.device.index or 0)
         rc = _lib.lib().octo_linear6d(ctx, C.byref(b), m, int(turns), C.c_void_p(st))

@@ -226,8 +226,7 @@ class Linear6DSpec:
 
     def to_c(self) -> _lib.OctoElement:
         e = _element(_lib.ELEM_LINEAR6D)
-        for k, v in enumerate(self.matrix):
-            e.p[k] = v
+        e.p[:36] = self.matrix
         return e
 
 
