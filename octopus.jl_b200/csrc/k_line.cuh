@@ -7,6 +7,10 @@
 // read through the constant bank.  Coordinates of either storage type are widened to FP64 on load and
 // rounded once on store; all element arithmetic is FP64.
 //
+// A map alone is bound by HBM, the lines by FP64 issue: block-diagonal maps run their 18 operations of 66 (kPlanar),
+// divisors that are constant or shared are divided by once (quotient), and Box-Muller's angle takes sincospi.  Both
+// rings' lines of a production turn (2.56M + 1.024M particles, 21 elements, four launches): 371 -> 308 us.
+//
 // Per-element constants that the reference evaluates per particle but that depend only on parameters
 // (cos / sin / tan of the boost angle, 1/sqrt of the coupling determinant, the crab harmonics' i kcc,
 // the Philox keys of the six radiation components) are evaluated once on the host with the same
@@ -36,11 +40,15 @@ constexpr int kRadDamping = 1, kRadExcitation = 2;
 constexpr int kZeroZeta = 4, kZeroEta = 8, kZeroR = 16;
 // Thin crab cavity: some harmonics had zero strengths in both planes and were dropped on the host.
 constexpr int kCrabDropped = 1;
+// Linear6D: every entry outside the three 2x2 plane blocks is zero (a map without coupling or dispersion).  The 24
+// products with them are zeros on finite coordinates, so such a particle runs the blocks alone, with the same result up
+// to the sign of a zero; a particle with a non-finite coordinate runs the whole matrix.
+constexpr int kPlanar = 1;
 
 // One compiled element.  a[] layout per kind:
 //   Linear6D   a[0..35] row-major matrix
-//   crab       a[h] i kcc, a[8+h] strengthX, a[16+h] strengthY, a[24+h] phase (h < n)
-//   boost      a[0] cos, a[1] sin, a[2] tan of the half crossing angle
+//   crab       a[h] i kcc, a[8+h] strengthX, a[16+h] strengthY, a[24+h] phase (h < n); rec[h] 1 / (i kcc), h < 6
+//   boost      a[0] cos, a[1] sin, a[2] tan of the half crossing angle; rec[0] 1 / cos, rec[1] 1 / cos^2
 //   chrom      a[0..1] xi, a[2..3] beta, a[4..5] alpha, a[6..7] gamma, a[8..11] zeta, a[12..15] eta,
 //              a[16..19] R, a[20] 1/sqrt(1 + r1 r4 - r2 r3)
 //   rad        a[0..2] damping, a[3..11] excitation, a[12..15] zeta, a[16..19] eta, a[20..23] R, a[24] g;
@@ -49,7 +57,10 @@ constexpr int kCrabDropped = 1;
 struct LineOp {
     int kind, n, flags, pad;
     double a[36];
-    unsigned long long key[6];
+    union {
+        unsigned long long key[6];
+        double rec[6];
+    };
 };
 struct LineProgram {
     int nops, rng, turns, pad;
@@ -120,8 +131,26 @@ __device__ __forceinline__ void xy_coupling_inv_a(Coords &c, const double *r, do
     c.py = g * (r[2] * x0 + r[3] * px0 + py0);
 }
 
-__device__ __forceinline__ void linear6d(Coords &c, const double *m) {
+__device__ __forceinline__ bool all_finite6(const Coords &c) { return isfinite(c.x + c.px + c.y + c.py + c.z + c.pz); }
+
+// x / d as the division rounds it, rd = 1 / d rounded: a product, its residual and one correction, where the division
+// makes its own reciprocal each time.  A quotient that overflows or is not a number stays what the product is.
+__device__ __forceinline__ double quotient(double x, double d, double rd) {
+    const double q = x * rd, r = fma(-q, d, x);
+    return r == r ? fma(r, rd, q) : q;
+}
+
+__device__ __forceinline__ void linear6d(Coords &c, const double *m, int flags) {
     const double a = c.x, b = c.px, d = c.y, e = c.py, f = c.z, h = c.pz;
+    if ((flags & kPlanar) && all_finite6(c)) {
+        c.x = m[0] * a + m[1] * b;
+        c.px = m[6] * a + m[7] * b;
+        c.y = m[14] * d + m[15] * e;
+        c.py = m[20] * d + m[21] * e;
+        c.z = m[28] * f + m[29] * h;
+        c.pz = m[34] * f + m[35] * h;
+        return;
+    }
     c.x = m[0] * a + m[1] * b + m[2] * d + m[3] * e + m[4] * f + m[5] * h;
     c.px = m[6] * a + m[7] * b + m[8] * d + m[9] * e + m[10] * f + m[11] * h;
     c.y = m[12] * a + m[13] * b + m[14] * d + m[15] * e + m[16] * f + m[17] * h;
@@ -141,8 +170,13 @@ __device__ __forceinline__ void crab_cavity(Coords &c, const LineOp &op) {
         double s, co;
         sincos(ikcc * c.z + op.a[24 + h], &s, &co);
         const double sx = op.a[8 + h], sy = op.a[16 + h];
-        dpx -= sx * s / ikcc;
-        dpy -= sy * s / ikcc;
+        if (h < 6) {
+            dpx -= quotient(sx * s, ikcc, op.rec[h]);
+            dpy -= quotient(sy * s, ikcc, op.rec[h]);
+        } else {
+            dpx -= sx * s / ikcc;
+            dpy -= sy * s / ikcc;
+        }
         dpz -= (sx * c.x + sy * c.y) * co;
     }
     if (op.flags & kCrabDropped) {
@@ -156,22 +190,20 @@ __device__ __forceinline__ void crab_cavity(Coords &c, const LineOp &op) {
     c.pz += dpz;
 }
 
-__device__ __forceinline__ bool all_finite6(const Coords &c) { return isfinite(c.x + c.px + c.y + c.py + c.z + c.pz); }
-
 // LorentzBoost and RevLorentzBoost (lorentz_boost.jl:128-161), Hirata's crossing-angle transformation.
-__device__ __forceinline__ void boost(Coords &c, double ca, double sa, double ta) {
+__device__ __forceinline__ void boost(Coords &c, double ca, double sa, double ta, double rca, double rca2) {
     const double x0 = c.x, px0 = c.px, y0 = c.y, py0 = c.py, z0 = c.z, pz0 = c.pz;
     const double ps0 = sqrt((1.0 + pz0) * (1.0 + pz0) - px0 * px0 - py0 * py0);
     const double h0 = 1.0 + pz0 - ps0;
-    const double py1 = py0 / ca;
-    const double h1 = h0 / (ca * ca);
-    const double px1 = px0 / ca - h1 * sa;
+    const double py1 = quotient(py0, ca, rca);
+    const double h1 = quotient(h0, ca * ca, rca2);
+    const double px1 = quotient(px0, ca, rca) - h1 * sa;
     const double pz1 = pz0 - px1 * sa;
     const double ps1 = 1.0 + pz1 - h1;
-    const double ds = x0 * sa;
-    c.x = x0 + z0 * ta + px1 / ps1 * ds;
-    c.y = y0 + py1 / ps1 * ds;
-    c.z = z0 / ca - h1 / ps1 * ds;
+    const double ds = x0 * sa, rps = 1.0 / ps1;
+    c.x = x0 + z0 * ta + quotient(px1, ps1, rps) * ds;
+    c.y = y0 + quotient(py1, ps1, rps) * ds;
+    c.z = quotient(z0, ca, rca) - quotient(h1, ps1, rps) * ds;
     c.px = px1;
     c.py = py1;
     c.pz = pz1;
@@ -180,10 +212,11 @@ __device__ __forceinline__ void rev_boost(Coords &c, double ca, double sa) {
     const double x0 = c.x, px0 = c.px, y0 = c.y, py0 = c.py, z0 = c.z, pz0 = c.pz;
     const double ps0 = sqrt((1.0 + pz0) * (1.0 + pz0) - px0 * px0 - py0 * py0);
     const double h0 = 1.0 + pz0 - ps0;
+    const double rps = 1.0 / ps0;
     double x1 = x0 - z0 * sa;
-    x1 = x1 / (1.0 + (px0 + h0 * sa) * sa / ps0);
-    c.z = (z0 + h0 / ps0 * x1 * sa) * ca;
-    c.y = y0 - py0 / ps0 * x1 * sa;
+    x1 = x1 / (1.0 + quotient((px0 + h0 * sa) * sa, ps0, rps));
+    c.z = (z0 + quotient(h0, ps0, rps) * x1 * sa) * ca;
+    c.y = y0 - quotient(py0, ps0, rps) * x1 * sa;
     c.pz = pz0 + px0 * sa;
     c.px = (px0 + h0 * sa) * ca;
     c.py = py0 * ca;
@@ -254,7 +287,7 @@ __device__ __forceinline__ void rad_plane(double &q, double &p, const double *e,
     const double u2 = line_uniform(rng, k2, particle, turn, smix_tp);
     const double rr = sqrt(-2.0 * log(u1));
     double s, co;
-    sincos(6.283185307179586476925286766559 * u2, &s, &co);
+    sincospi(2.0 * u2, &s, &co);  // of 2 pi u2 unrounded: its reduction is exact and a few instructions
     const double n1 = rr * co, n2 = rr * s;
     q += e[0] * n1;
     p += e[1] * n2 + e[2] * n1;
@@ -318,9 +351,9 @@ __global__ void __launch_bounds__(256) k_track_line(R *__restrict__ x, R *__rest
                 if (k >= P.nops) break;
                 const LineOp &op = P.op[k];
                 switch (op.kind) {
-                    case kElemLinear6D: linear6d(c, op.a); break;
+                    case kElemLinear6D: linear6d(c, op.a, op.flags); break;
                     case kElemCrab: crab_cavity(c, op); break;
-                    case kElemBoost: boost(c, op.a[0], op.a[1], op.a[2]); break;
+                    case kElemBoost: boost(c, op.a[0], op.a[1], op.a[2], op.rec[0], op.rec[1]); break;
                     case kElemRevBoost: rev_boost(c, op.a[0], op.a[1]); break;
                     case kElemChrom: chromaticity(c, op.a, op.flags); break;
                     case kElemRad: lumped_rad(c, op, P.rng, particle, turn, smix_tp); break;

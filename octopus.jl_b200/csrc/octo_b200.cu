@@ -2211,7 +2211,11 @@ int compile_line_op(const octo_element &e, int rng, uint64_t seed, LineOp &op, s
                 msg = b;
                 return OCTO_ERR_ARG;
             }
-            for (int k = 0; k < 36; ++k) op.a[k] = p[k];
+            op.flags = kPlanar;
+            for (int k = 0; k < 36; ++k) {
+                op.a[k] = p[k];
+                if (k / 12 != k % 6 / 2 && p[k] != 0.0) op.flags = 0;  // an entry outside the plane blocks
+            }
             return OCTO_OK;
         }
         case OCTO_ELEM_THIN_CRAB_CAVITY: {
@@ -2237,6 +2241,7 @@ int compile_line_op(const octo_element &e, int rng, uint64_t seed, LineOp &op, s
                 op.a[8 + op.n] = p[1 + h];
                 op.a[16 + op.n] = p[9 + h];
                 op.a[24 + op.n] = p[17 + h];
+                if (op.n < 6) op.rec[op.n] = 1.0 / op.a[op.n];
                 ++op.n;
             }
             return OCTO_OK;
@@ -2249,6 +2254,8 @@ int compile_line_op(const octo_element &e, int rng, uint64_t seed, LineOp &op, s
             op.a[0] = c;
             op.a[1] = s;
             op.a[2] = s / c;
+            op.rec[0] = 1.0 / c;
+            op.rec[1] = 1.0 / (c * c);
             return OCTO_OK;
         }
         case OCTO_ELEM_CHROMATICITY_KICK: {
