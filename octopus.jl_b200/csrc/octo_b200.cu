@@ -1459,7 +1459,12 @@ void CollideJob::run() {
         double slice_bytes = 0.0, src_bytes = 0.0, fld_bytes = 0.0;
         for (int t = F.t0; t < F.t0 + F.nt; t += 2) slice_bytes += (double)(tasks[t].src_n + tasks[t].fld_n);
         for (int t = F.t0; t < F.t0 + F.nt; ++t) { src_bytes += (double)tasks[t].src_n; fld_bytes += (double)tasks[t].fld_n; }
-        const unsigned bps = (unsigned)std::max<long long>(1, std::min<long long>(kMaxBoundBlocks, (F.maxsrc + 2047) / 2048));
+        // blocks per slice of the bounds passes: 2048 particles each, fewer (down to one a thread) where that leaves
+        // less than four blocks per SM -- the extrema do not depend on the split; the hybrid's moments and :sigma's
+        // sums do, so theirs stays
+        const long long coarse = std::max<long long>(1, 2 * npf * ((F.maxsrc + 2047) / 2048)), want = 4LL * c->num_sms;
+        const long long per = gaussian || c->dopt.grid_extent || coarse >= want ? 2048 : std::max<long long>(256, 2048 * coarse / want);
+        const unsigned bps = (unsigned)std::max<long long>(1, std::min<long long>(kMaxBoundBlocks, (F.maxsrc + per - 1) / per));
         bool union_first = false;
         for (int t = F.t0; t < F.t0 + F.nt; ++t) union_first = union_first || tasks[t].ub_first;
         if (union_first) {
@@ -1501,7 +1506,9 @@ void CollideJob::run() {
                 PhaseScope ps(c, OCTO_PHASE_LUMINOSITY, c->lum_stream, 2, slice_bytes * 4 * rsz);
                 // uniform blocks per side: this stream runs beside the front's deposit and convolution and wants
                 // parallelism (blocks in proportion to each side's slice, sized to whole waves, measured slower)
-                unsigned bpp = (unsigned)std::max<long long>(1, std::min<long long>(8, (F.maxlum + 32767) / 32768));
+                // 32,768 particles each, fewer (down to 2,048) where the front would leave SMs without a block
+                const long long lper = std::max<long long>(2048, std::min<long long>(32768, 2 * F.nl * F.maxlum / c->num_sms));
+                unsigned bpp = (unsigned)std::max<long long>(1, std::min<long long>(8, (F.maxlum + lper - 1) / lper));
                 with_real(fp32, [&](auto r) {
                     launch_method(lmethod, [&](auto M) {
                         launch_pdl(k_lum_deposit<decltype(r), decltype(M)::value>, dim3(bpp, 2 * F.nl), 1024, lum_bytes, c->lum_stream, 
