@@ -46,7 +46,8 @@ struct Cnn {
     // backward scratch
     DevBuf<bf16> g, gt, colt;
     DevBuf<float> fa, dc, ds1, ds2, ds3, part, splitbuf;
-    DevBuf<double> loss_part;
+    DevBuf<float> bpart;         // bias-gradient block sums
+    DevBuf<double> loss_part, wpart;
     PinBuf<double> h_loss;
     long long part_floats = 0;
     int adam_t = 0;
@@ -109,6 +110,8 @@ struct Cnn {
         }
         part.ensure(pmax);
         part_floats = pmax;
+        bpart.ensure(kBiasBlocks * 256);
+        wpart.ensure(kMaskBlocks);
         loss_part.ensure(2 * 1024);
         h_loss.ensure(2 * 1024);
         CK(cudaMalloc(&err, sizeof(int)));
@@ -122,6 +125,8 @@ struct Cnn {
         for (DevBuf<bf16> *b : {&x0, &a0, &s1, &p1, &a2, &s2, &p2, &a4, &s3, &p3, &b6, &u3, &d7, &u2, &d8, &u1, &d9, &g, &gt, &colt})
             b->release();
         for (DevBuf<float> *b : {&out, &fa, &dc, &ds1, &ds2, &ds3, &part, &splitbuf}) b->release();
+        bpart.release();
+        wpart.release();
         loss_part.release();
         h_loss.release();
         if (err) cudaFree(err);
@@ -186,11 +191,11 @@ struct Cnn {
     }
 
     void pool(const bf16 *in, bf16 *o, int B, int level, int C, cudaStream_t st) {
-        const long long n = ml(level + 1, B) * C;
+        const long long n = ml(level + 1, B) * (C / 8);
         launch_pdl(k_cnn_pool, ew_blocks(n), 256, 0, st, in, o, B, hl(level), wl(level), C);
     }
     void upcat(const bf16 *coarse, const bf16 *skip, bf16 *o, int B, int level, int Cu, int Cs, cudaStream_t st) {
-        const long long n = ml(level, B) * (Cu + Cs);
+        const long long n = ml(level, B) * ((Cu + Cs) / 8);
         launch_pdl(k_cnn_upcat, ew_blocks(n), 256, 0, st, coarse, skip, o, B, hl(level), wl(level), Cu, Cs);
     }
 
@@ -235,14 +240,24 @@ struct Cnn {
         gemm_conv(L_HEAD, d9.p, B, nullptr, out.p, st);
     }
 
+    // out[(tap * C + c)][m] of an NHWC tensor (TAPS = 1: its transpose), 32 channels a block or 8
+    template <int TAPS>
+    void im2col_t(const bf16 *in, bf16 *o, long long M, int hh, int ww, int C, long long ld, cudaStream_t st) {
+        if (C % 32 == 0)
+            launch_pdl(k_cnn_im2col_t<32, TAPS>, dim3((unsigned)((ld + 63) / 64), C / 32, TAPS), kIm2colThreads, 0, st, in, o,
+                       M, hh, ww, C, ld);
+        else
+            launch_pdl(k_cnn_im2col_t<8, TAPS>, dim3((unsigned)((ld + 255) / 256), C / 8, TAPS), kIm2colThreads, 0, st, in, o,
+                       M, hh, ww, C, ld);
+    }
+
     // Weight and bias gradients of layer l from its input activation and the bf16 output gradient in g.
     void wgrad(int l, const bf16 *in, int B, cudaStream_t st) {
         const LayerSpec &L = kLayers[l];
         const long long M = ml(L.level, B), ld = round8(M);
         const int hh = hl(L.level), ww = wl(L.level);
-        launch_pdl(k_cnn_transpose, dim3((unsigned)((ld + 31) / 32), (unsigned)((L.cout + 31) / 32)), dim3(32, 8), 0, st,
-                   (const bf16 *)g.p, gt.p, M, L.cout, ld);
-        launch_pdl(k_cnn_im2col_t, ew_blocks(9LL * L.cin * ld), 256, 0, st, in, colt.p, B, hh, ww, L.cin, ld);
+        im2col_t<1>((const bf16 *)g.p, gt.p, M, hh, ww, L.cout, ld, st);
+        im2col_t<9>(in, colt.p, M, hh, ww, L.cin, ld, st);
         const int splits = wgrad_splits(l, B);
         GemmArgs a{};
         a.M = 9 * L.cin; a.N = L.cout; a.K = (int)ld;
@@ -255,8 +270,9 @@ struct Cnn {
         const int used = (int)((chunks * kBK + a.k_per_split - 1) / a.k_per_split);
         launch_gemm(a, used, st);
         const long long n = (long long)a.M * L.cout;
-        launch_pdl(k_cnn_wgrad_reduce, ew_blocks(n), 256, 0, st, (const float *)part.p, used, a.M, L.cout, grad.p + woff[l]);
-        launch_pdl(k_cnn_bias_grad, L.cout, 256, 0, st, (const bf16 *)g.p, M, L.cout, grad.p + boff[l]);
+        launch_pdl(k_cnn_bias_part, kBiasBlocks, 256, 0, st, (const bf16 *)g.p, M, L.cout, bpart.p);
+        launch_pdl(k_cnn_wgrad_reduce, ew_blocks(8 * (n + 31 + L.cout)), 256, 0, st, (const float *)part.p, used, a.M, L.cout,
+                   grad.p + woff[l], (const float *)bpart.p, grad.p + boff[l]);
     }
 
     // Input gradient of layer l (fp32, into fa) from the bf16 output gradient in g.
@@ -271,17 +287,18 @@ struct Cnn {
         launch_gemm(a, 1, st);
     }
     void relu_grad(const float *dy, const bf16 *y, long long n, cudaStream_t st) {
-        launch_pdl(k_cnn_relu_grad, ew_blocks(n), 256, 0, st, dy, y, g.p, n);
+        launch_pdl(k_cnn_relu_grad, ew_blocks(n / 8), 256, 0, st, dy, y, g.p, n);
     }
 
     // Loss of the last forward pass against target ([M0][2]) with per-pixel weights mask (null = 1),
     // normalised by the total weight; then the gradients of every parameter into `grad`.  Returns the
     // partial-sum count; the host folds loss_part.
-    int backward(int B, const float *target, const float *mask, double weight_total, cudaStream_t st) {
+    int backward(int B, const float *target, const float *mask, cudaStream_t st) {
         const long long M0 = ml(0, B), M1 = ml(1, B), M2 = ml(2, B), M3 = ml(3, B);
         const int nblk = (int)std::min<long long>(1024, (M0 + 255) / 256);
-        const float scale = (float)(1.0 / (2.0 * std::max(weight_total, 1e-300)));  // mean over 2 channels
-        launch_pdl(k_cnn_loss, nblk, 256, 0, st, (const float *)out.p, target, mask, M0, scale, g.p, loss_part.p);
+        if (mask) launch_pdl(k_cnn_mask_sum, kMaskBlocks, 256, 0, st, mask, M0, wpart.p);
+        launch_pdl(k_cnn_loss, nblk, 256, 0, st, (const float *)out.p, target, mask, M0, (const double *)wpart.p, g.p,
+                   loss_part.p);
         // head
         wgrad(L_HEAD, d9.p, B, st);
         dgrad(L_HEAD, B, st);
@@ -289,25 +306,25 @@ struct Cnn {
         // d1: input [up(d2), s1]
         wgrad(L_D1, u1.p, B, st);
         dgrad(L_D1, B, st);
-        launch_pdl(k_cnn_upcat_adj, ew_blocks(M1 * 32 + M0 * 32), 256, 0, st, (const float *)fa.p, dc.p, ds1.p, B, hl(0), wl(0), 32,
-                   32, 0);
+        launch_pdl(k_cnn_upcat_adj, ew_blocks(M1 * 4 + M0 * 4), 256, 0, st, (const float *)fa.p, dc.p, ds1.p, B, hl(0), wl(0), 32,
+                   32);
         relu_grad(dc.p, d8.p, M1 * 32, st);
         // d2: input [up(d3), s2]
         wgrad(L_D2, u2.p, B, st);
         dgrad(L_D2, B, st);
-        launch_pdl(k_cnn_upcat_adj, ew_blocks(M2 * 64 + M1 * 64), 256, 0, st, (const float *)fa.p, dc.p, ds2.p, B, hl(1), wl(1), 64,
-                   64, 0);
+        launch_pdl(k_cnn_upcat_adj, ew_blocks(M2 * 8 + M1 * 8), 256, 0, st, (const float *)fa.p, dc.p, ds2.p, B, hl(1), wl(1), 64,
+                   64);
         relu_grad(dc.p, d7.p, M2 * 64, st);
         // d3: input [up(b), s3]
         wgrad(L_D3, u3.p, B, st);
         dgrad(L_D3, B, st);
-        launch_pdl(k_cnn_upcat_adj, ew_blocks(M3 * 128 + M2 * 128), 256, 0, st, (const float *)fa.p, dc.p, ds3.p, B, hl(2), wl(2),
-                   128, 128, 0);
+        launch_pdl(k_cnn_upcat_adj, ew_blocks(M3 * 16 + M2 * 16), 256, 0, st, (const float *)fa.p, dc.p, ds3.p, B, hl(2), wl(2),
+                   128, 128);
         relu_grad(dc.p, b6.p, M3 * 128, st);
         // b: input pool(s3)
         wgrad(L_B, p3.p, B, st);
         dgrad(L_B, B, st);
-        launch_pdl(k_cnn_pool_adj_add, ew_blocks(M2 * 128), 256, 0, st, (const float *)fa.p, ds3.p, B, hl(2), wl(2), 128);
+        launch_pdl(k_cnn_pool_adj_add, ew_blocks(M2 * 16), 256, 0, st, (const float *)fa.p, ds3.p, B, hl(2), wl(2), 128);
         relu_grad(ds3.p, s3.p, M2 * 128, st);
         // e3b, e3a
         wgrad(L_E3B, a4.p, B, st);
@@ -315,7 +332,7 @@ struct Cnn {
         relu_grad(fa.p, a4.p, M2 * 128, st);
         wgrad(L_E3A, p2.p, B, st);
         dgrad(L_E3A, B, st);
-        launch_pdl(k_cnn_pool_adj_add, ew_blocks(M1 * 64), 256, 0, st, (const float *)fa.p, ds2.p, B, hl(1), wl(1), 64);
+        launch_pdl(k_cnn_pool_adj_add, ew_blocks(M1 * 8), 256, 0, st, (const float *)fa.p, ds2.p, B, hl(1), wl(1), 64);
         relu_grad(ds2.p, s2.p, M1 * 64, st);
         // e2b, e2a
         wgrad(L_E2B, a2.p, B, st);
@@ -323,7 +340,7 @@ struct Cnn {
         relu_grad(fa.p, a2.p, M1 * 64, st);
         wgrad(L_E2A, p1.p, B, st);
         dgrad(L_E2A, B, st);
-        launch_pdl(k_cnn_pool_adj_add, ew_blocks(M0 * 32), 256, 0, st, (const float *)fa.p, ds1.p, B, hl(0), wl(0), 32);
+        launch_pdl(k_cnn_pool_adj_add, ew_blocks(M0 * 4), 256, 0, st, (const float *)fa.p, ds1.p, B, hl(0), wl(0), 32);
         relu_grad(ds1.p, s1.p, M0 * 32, st);
         // e1b, e1a
         wgrad(L_E1B, a0.p, B, st);

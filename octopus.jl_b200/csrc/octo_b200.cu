@@ -3225,17 +3225,9 @@ int32_t octo_cnn_train_step(octo_cnn *c, const void *input, const float *target,
         CK(cudaSetDevice(N.device));
         cudaStream_t st = (cudaStream_t)stream;
         const long long M0 = N.ml(0, batch);
-        double wt = (double)M0;
-        if (mask) {  // the loss is normalised by the total weight
-            std::vector<float> hm((size_t)M0);
-            CK(cudaMemcpyAsync(hm.data(), mask, sizeof(float) * M0, cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
-            wt = 0.0;
-            for (float v : hm) wt += v;
-        }
         CK(cudaMemcpyAsync(N.x0.p, input, sizeof(nn::bf16) * M0 * nn::kCnnIn, cudaMemcpyDeviceToDevice, st));
         N.forward(batch, st);
-        const int nblk = N.backward(batch, target, mask, wt, st);
+        const int nblk = N.backward(batch, target, mask, st);
         if (loss) {
             CK(cudaMemcpyAsync(N.h_loss.p, N.loss_part.p, sizeof(double) * 2 * nblk, cudaMemcpyDeviceToHost, st));
         }
@@ -3243,8 +3235,11 @@ int32_t octo_cnn_train_step(octo_cnn *c, const void *input, const float *target,
         if (update) N.adam(lr, st);
         const int rc = cnn_status(c, st);
         if (loss) {
-            double se = 0.0;
-            for (int b = 0; b < nblk; ++b) se += N.h_loss.p[2 * b];
+            double se = 0.0, wt = 0.0;
+            for (int b = 0; b < nblk; ++b) {
+                se += N.h_loss.p[2 * b];
+                wt += N.h_loss.p[2 * b + 1];
+            }
             *loss = se / (2.0 * std::max(wt, 1e-300));
         }
         return rc;
