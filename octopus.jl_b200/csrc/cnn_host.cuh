@@ -153,13 +153,30 @@ struct Cnn {
         weights_dirty = false;
     }
 
-    // A 3x3 convolution layer as one tensor-core GEMM.  Layers with too few output tiles to fill the GPU (the
-    // coarse levels) split K over more CTAs; their fp32 partials are summed in a fixed order by the
-    // bias / ReLU / bf16 epilogue kernel.
+    // A 3x3 convolution layer: by bands of the image (k_conv.cuh), or where no band fits a CTA as one im2col GEMM,
+    // whose layers with too few output tiles to fill the GPU (the coarse levels) split K over more CTAs, their fp32
+    // partials summed in a fixed order by the bias / ReLU / bf16 epilogue kernel.
     // skip != null: the layer's input is [nearest-upsampled in (cu channels), skip] (a decoder level), read
-    // by the GEMM directly instead of a materialised concatenation.
-    void gemm_conv(int l, const bf16 *in, int B, bf16 *out_bf, float *out_f, cudaStream_t st, const bf16 *skip = nullptr,
-                   int cu = 0) {
+    // directly instead of a materialised concatenation.  pooled != null: the layer's input is the 2x2 average of in;
+    // a GEMM takes it from pooled, which this then fills.
+    void conv(int l, const bf16 *in, int B, bf16 *out_bf, float *out_f, cudaStream_t st, const bf16 *skip = nullptr,
+              int cu = 0, bf16 *pooled = nullptr) {
+        const LayerSpec &L = kLayers[l];
+        ConvArgs c{};
+        c.in = in; c.skip = skip; c.Cu = cu; c.pool = pooled != nullptr;
+        c.H = hl(L.level); c.W = wl(L.level); c.C = L.cin;
+        c.w = w[l].p; c.N = L.cout;
+        c.bias = master.p + boff[l]; c.relu = L.relu;
+        c.out_bf16 = out_bf; c.out = out_f;
+        c.error = err;
+        if (launch_conv(c, B, st)) return;
+        if (pooled) {
+            pool(in, pooled, B, L.level - 1, L.cin, st);
+            in = pooled;
+        }
+        gemm_conv(l, in, B, out_bf, out_f, st, skip, cu);
+    }
+    void gemm_conv(int l, const bf16 *in, int B, bf16 *out_bf, float *out_f, cudaStream_t st, const bf16 *skip, int cu) {
         const LayerSpec &L = kLayers[l];
         GemmArgs a{};
         a.M = (int)ml(L.level, B); a.N = L.cout; a.K = 9 * L.cin;
@@ -205,39 +222,36 @@ struct Cnn {
     void forward(int B, cudaStream_t st, bool materialize = true) {
         if (weights_dirty) refresh_weights(st);
         if (!materialize) {
-            gemm_conv(L_E1A, x0.p, B, a0.p, nullptr, st);
-            gemm_conv(L_E1B, a0.p, B, s1.p, nullptr, st);
-            pool(s1.p, p1.p, B, 0, 32, st);
-            gemm_conv(L_E2A, p1.p, B, a2.p, nullptr, st);
-            gemm_conv(L_E2B, a2.p, B, s2.p, nullptr, st);
-            pool(s2.p, p2.p, B, 1, 64, st);
-            gemm_conv(L_E3A, p2.p, B, a4.p, nullptr, st);
-            gemm_conv(L_E3B, a4.p, B, s3.p, nullptr, st);
-            pool(s3.p, p3.p, B, 2, 128, st);
-            gemm_conv(L_B, p3.p, B, b6.p, nullptr, st);
-            gemm_conv(L_D3, b6.p, B, d7.p, nullptr, st, s3.p, 128);
-            gemm_conv(L_D2, d7.p, B, d8.p, nullptr, st, s2.p, 64);
-            gemm_conv(L_D1, d8.p, B, d9.p, nullptr, st, s1.p, 32);
-            gemm_conv(L_HEAD, d9.p, B, nullptr, out.p, st);
+            conv(L_E1A, x0.p, B, a0.p, nullptr, st);
+            conv(L_E1B, a0.p, B, s1.p, nullptr, st);
+            conv(L_E2A, s1.p, B, a2.p, nullptr, st, nullptr, 0, p1.p);
+            conv(L_E2B, a2.p, B, s2.p, nullptr, st);
+            conv(L_E3A, s2.p, B, a4.p, nullptr, st, nullptr, 0, p2.p);
+            conv(L_E3B, a4.p, B, s3.p, nullptr, st);
+            conv(L_B, s3.p, B, b6.p, nullptr, st, nullptr, 0, p3.p);
+            conv(L_D3, b6.p, B, d7.p, nullptr, st, s3.p, 128);
+            conv(L_D2, d7.p, B, d8.p, nullptr, st, s2.p, 64);
+            conv(L_D1, d8.p, B, d9.p, nullptr, st, s1.p, 32);
+            conv(L_HEAD, d9.p, B, nullptr, out.p, st);
             return;
         }
-        gemm_conv(L_E1A, x0.p, B, a0.p, nullptr, st);
-        gemm_conv(L_E1B, a0.p, B, s1.p, nullptr, st);
+        conv(L_E1A, x0.p, B, a0.p, nullptr, st);
+        conv(L_E1B, a0.p, B, s1.p, nullptr, st);
         pool(s1.p, p1.p, B, 0, 32, st);
-        gemm_conv(L_E2A, p1.p, B, a2.p, nullptr, st);
-        gemm_conv(L_E2B, a2.p, B, s2.p, nullptr, st);
+        conv(L_E2A, p1.p, B, a2.p, nullptr, st);
+        conv(L_E2B, a2.p, B, s2.p, nullptr, st);
         pool(s2.p, p2.p, B, 1, 64, st);
-        gemm_conv(L_E3A, p2.p, B, a4.p, nullptr, st);
-        gemm_conv(L_E3B, a4.p, B, s3.p, nullptr, st);
+        conv(L_E3A, p2.p, B, a4.p, nullptr, st);
+        conv(L_E3B, a4.p, B, s3.p, nullptr, st);
         pool(s3.p, p3.p, B, 2, 128, st);
-        gemm_conv(L_B, p3.p, B, b6.p, nullptr, st);
+        conv(L_B, p3.p, B, b6.p, nullptr, st);
         upcat(b6.p, s3.p, u3.p, B, 2, 128, 128, st);
-        gemm_conv(L_D3, u3.p, B, d7.p, nullptr, st);
+        conv(L_D3, u3.p, B, d7.p, nullptr, st);
         upcat(d7.p, s2.p, u2.p, B, 1, 64, 64, st);
-        gemm_conv(L_D2, u2.p, B, d8.p, nullptr, st);
+        conv(L_D2, u2.p, B, d8.p, nullptr, st);
         upcat(d8.p, s1.p, u1.p, B, 0, 32, 32, st);
-        gemm_conv(L_D1, u1.p, B, d9.p, nullptr, st);
-        gemm_conv(L_HEAD, d9.p, B, nullptr, out.p, st);
+        conv(L_D1, u1.p, B, d9.p, nullptr, st);
+        conv(L_HEAD, d9.p, B, nullptr, out.p, st);
     }
 
     // out[(tap * C + c)][m] of an NHWC tensor (TAPS = 1: its transpose), 32 channels a block or 8
@@ -278,6 +292,12 @@ struct Cnn {
     // Input gradient of layer l (fp32, into fa) from the bf16 output gradient in g.
     void dgrad(int l, int B, cudaStream_t st) {
         const LayerSpec &L = kLayers[l];
+        ConvArgs c{};  // the convolution of g with the flipped, transposed weights
+        c.in = g.p; c.H = hl(L.level); c.W = wl(L.level); c.C = L.cout;
+        c.w = wf[l].p; c.N = L.cin;
+        c.out = fa.p;
+        c.error = err;
+        if (launch_conv(c, B, st)) return;
         GemmArgs a{};
         a.M = (int)ml(L.level, B); a.N = L.cin; a.K = 9 * L.cout;
         a.A = g.p; a.a_mode = 1; a.H = hl(L.level); a.W = wl(L.level); a.C = L.cout;

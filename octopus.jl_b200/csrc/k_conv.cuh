@@ -1,0 +1,240 @@
+// 3x3 / padding-1 convolution of an NHWC bf16 tensor on the fifth-generation tensor cores, one band of output rows of
+// one image a CTA: the forward layers and the input gradients of the learned field correction's network.
+//
+// The band's input rows (with their halo, zero-padded to W + 2 columns) are brought into shared memory once, as one
+// plane of 16-byte pixels per 8 channels.  Pixel p of a plane lies 16 p bytes after its start, which is the canonical
+// no-swizzle K-major layout with 8-row groups 128 bytes apart, so the A operand of a tap is the same planes read from
+// a start address 16 bytes x (dy (W + 2) + dx) further on: no im2col is written or loaded.  Row o = y (W + 2) + x of
+// the product is output pixel (y, x); the two columns x >= W of each row are computed and dropped (4 % at W = 48).
+// The weights of the CTA's NB output channels lie beside it in the same form.  Warp t's first lane issues every
+// tcgen05.mma (M = 128 pixels, N = NB, K = 16) of tile t into TMEM and commits once; an instruction's operands are two
+// additions away from the one before (rebuilt descriptors made the issuing lane the layer's longest part).
+//   C = 8: the two K halves of an instruction are two neighbouring taps (the same plane 16 bytes further on).
+//   pool: the input is read as the 2x2 average of a tensor of twice the height and width.
+//   skip: the input is [nearest-upsampled in (Cu channels), skip] (a decoder level).
+// Bound by latency: a layer is a few microseconds of loads, instructions and stores between two launches.  The im2col
+// GEMM (k_umma.cuh) reads every input nine times in K chunks that wait for one another: a forward pass over 20 planes of
+// 48 x 48 took 304 us with it (split-K folds and pools included) and takes 177 us; a batch-64 training step 2.01 and 1.57 ms.
+//
+// The mbarrier wait is bounded (about one second of the global timer); on expiry the kernel records OCTO_ERR_TIMEOUT
+// in *error, frees its TMEM and returns.
+#pragma once
+#include <algorithm>
+
+#include "k_cnn.cuh"
+#include "k_umma.cuh"
+
+namespace octo {
+namespace nn {
+
+constexpr int kConvThreads = 256;
+
+struct ConvArgs {
+    const bf16 *in, *skip;   // skip: null, or [b][H][W][C - Cu] beside the upsampled in [b][H/2][W/2][Cu]
+    int Cu, pool;            // pool: in is [b][2H][2W][C]
+    int H, W, C;             // C = 8 or a multiple of 16; Cu a multiple of 8
+    const bf16 *w;           // [N][3][3][C]
+    int N;                   // output channels (row length of the output)
+    const float *bias;       // null: none
+    int relu;
+    bf16 *out_bf16;          // bf16 result, or null:
+    float *out;              // fp32 result
+    int *error;
+    // the split (conv_plan): rows a band, 128-row tiles a band, pixels of a plane (odd), TMEM columns
+    int R, tiles, plane, cols;
+};
+
+// Shared memory of a CTA: weights, then input planes.
+inline size_t conv_smem(int C, int nb, int plane) {
+    return (size_t)(C == 8 ? 12 : 9 * (C / 8)) * nb * 16 + (size_t)(C / 8) * plane * 16;
+}
+
+// Rows a band for B images at nb channels a CTA: the least of a launch's fixed latency per wave, the bytes each SM brings
+// in and the instructions it issues, over the bands that fit (half of TMEM, so that two CTAs share an SM, and 200 KB).
+// Returns that cost (about a microsecond a unit), 1e30 when none fits (very wide images: the im2col GEMM runs those).
+constexpr double kConvNone = 1e30;
+inline double conv_plan(ConvArgs &g, int B, int nb) {
+    if (g.C % 16 && g.C != 8) return kConvNone;
+    const int wp = g.W + 2, nblk = (g.N + nb - 1) / nb, steps = g.C == 8 ? 6 : 9 * (g.C / 16);
+    double best = kConvNone;
+    for (int R = 1; R <= g.H; ++R) {
+        const int tiles = (R * wp + 127) / 128;
+        if (tiles * nb > 256) break;
+        const int plane = (tiles * 128 + 2 * wp + 4) | 1;
+        const size_t smem = conv_smem(g.C, nb, plane);
+        if (smem > 200 * 1024) break;
+        int cols = 32;
+        while (cols < tiles * nb) cols *= 2;
+        const long long ctas = (long long)((g.H + R - 1) / R) * B * nblk;
+        const int res = (int)std::min<long long>({(long long)(225 * 1024 / (smem + 1024)), 512 / cols, 8});
+        const double per_sm = (double)((ctas + 147) / 148), waves = (double)((ctas + 148LL * res - 1) / (148LL * res));
+        const double cost = 4.0 * waves + per_sm * (smem * 8.3e-6 + 0.008 * tiles * steps * (nb / 16));
+        if (cost < best) {
+            best = cost;
+            g.R = R;
+            g.tiles = tiles;
+            g.plane = plane;
+            g.cols = cols;
+        }
+    }
+    return best;
+}
+
+template <int NB>
+__global__ void __launch_bounds__(kConvThreads) k_conv3(const __grid_constant__ ConvArgs g) {
+    static_assert(NB == 16 || NB == 32, "NB");
+    extern __shared__ __align__(1024) unsigned char g_umma_smem[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_flag;
+    __shared__ float sbias[NB];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int c8 = g.C / 8, n0 = blockIdx.z * NB, wp = g.W + 2;
+    const int y0 = blockIdx.x * g.R, rows = min(g.R, g.H - y0);
+    const int tiles = (rows * wp + 127) / 128, issuers = min(tiles, kConvThreads / 32);
+    const long long img = blockIdx.y;
+    const uint32_t sB = smem_u32(g_umma_smem), sA = sB + (uint32_t)((g.C == 8 ? 12 : 9 * c8) * NB * 16);
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&bar)), "r"(issuers));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        abort_flag = 0;
+    }
+    // weights and bias, before the wait on the previous kernel: they are written by k_cnn_weights and k_cnn_adam, which
+    // lie at least one whole kernel before it in the stream.  Chunk (tap, 8 channels) of output channel n: [chunk][n] of 16 bytes; for
+    // C = 8 the chunks of a row of taps are dx = 0, 1, 2 and one of zeros.  Two chunks of 16 channels a warp.
+    if (tid < NB) sbias[tid] = g.bias && n0 + tid < g.N ? g.bias[n0 + tid] : 0.f;
+    {
+        const int k8 = 9 * c8, chunks = g.C == 8 ? 12 : k8;
+        for (int i = tid; i < chunks * NB; i += kConvThreads) {  // an even number of chunks: C = 8 or C % 16 == 0
+            const int pair = i / (2 * NB), r = i - pair * 2 * NB, k = 2 * pair + (r & 1), n = r >> 1;
+            const int src = g.C == 8 ? (k >> 2) * 3 + (k & 3) : k;
+            const bool ok = n0 + n < g.N && (g.C != 8 || (k & 3) < 3);
+            cp_async16(sB + (uint32_t)((k * NB + n) * 16), ok ? g.w + ((long long)(n0 + n) * k8 + src) * 8 : g.w, ok ? 16 : 0);
+        }
+    }
+    pdl_wait();
+    pdl_release();
+    // TMEM only now: the previous kernel's CTAs have all ended and freed theirs, so none of them can be waiting for
+    // columns that this kernel holds while it waits for them
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(g.cols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    // input rows y0 - 1 .. y0 + rows, zero outside the image
+    {
+        const int Cs = g.C - g.Cu, count = (rows + 2) * wp * c8;
+        // C = 8 multiplies the pixel after the last by the chunk of zeros: it must be finite
+        if (g.C == 8 && tid == 0) cp_async16(sA + (uint32_t)((rows + 2) * wp * 16), g.in, 0);
+        for (int i = tid; i < count; i += kConvThreads) {
+            const int p = i / c8, k = i - p * c8, py = p / wp;
+            const int y = y0 - 1 + py, x = p - py * wp - 1, c = k * 8;
+            const uint32_t dst = sA + (uint32_t)((k * g.plane + p) * 16);
+            const bool in = y >= 0 && y < g.H && x >= 0 && x < g.W;
+            if (g.pool) {
+                float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                if (in) {
+                    const long long ld = 2LL * g.W * g.C;
+                    const bf16 *s = g.in + ((img * 2 * g.H + 2 * y) * 2 * g.W + 2 * x) * g.C + c;
+                    const Bf8 q0 = load_bf8(s), q1 = load_bf8(s + g.C), q2 = load_bf8(s + ld), q3 = load_bf8(s + ld + g.C);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) v[e] = 0.25f * (q0.v[e] + q1.v[e] + q2.v[e] + q3.v[e]);
+                }
+                store_bf8(reinterpret_cast<bf16 *>(g_umma_smem + (dst - sB)), v);
+                continue;
+            }
+            const bf16 *s = g.in;
+            if (in) {
+                if (!g.skip) s = g.in + ((img * g.H + y) * g.W + x) * g.C + c;
+                else if (c < g.Cu) s = g.in + ((img * (g.H / 2) + y / 2) * (g.W / 2) + x / 2) * g.Cu + c;
+                else s = g.skip + ((img * g.H + y) * g.W + x) * Cs + (c - g.Cu);
+            }
+            cp_async16(dst, s, in ? 16 : 0);
+        }
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const uint32_t tmem = tmem_slot;
+    if (warp < issuers && lane == 0) {
+        const uint32_t idesc = umma_idesc_bf16(NB);
+        const bool c_is_8 = g.C == 8;
+        const int per_tap = c_is_8 ? 2 : g.C / 16, taps = c_is_8 ? 3 : 9;
+        // both descriptors' upper words are the tile's constants; the lower words hold the address in 16-byte units
+        const uint64_t da0 = umma_desc(sA, c_is_8 ? 16u : (uint32_t)g.plane * 16u, 128), db0 = umma_desc(sB, NB * 16, 128);
+        const uint32_t ha = (uint32_t)(da0 >> 32), hb = (uint32_t)(db0 >> 32), stepA = c_is_8 ? 2u : 2u * (uint32_t)g.plane;
+        for (int t = warp; t < tiles; t += kConvThreads / 32) {
+            const uint32_t d = tmem + (uint32_t)(t * NB);
+            uint32_t b = (uint32_t)db0, acc = 0;
+            for (int tap = 0; tap < taps; ++tap) {
+                uint32_t a = (uint32_t)da0 + (uint32_t)(t * 128 + (c_is_8 ? tap * wp : (tap / 3) * wp + tap % 3));
+#pragma unroll 2
+                for (int k = 0; k < per_tap; ++k) {
+                    asm volatile(
+                        "{\n\t.reg .pred p;\n\t.reg .b64 x, y;\n\t"
+                        "setp.ne.b32 p, %6, 0;\n\t"
+                        "mov.b64 x, {%1, %2};\n\t"
+                        "mov.b64 y, {%3, %4};\n\t"
+                        "tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %5, p;\n\t}"
+                        :
+                        : "r"(d), "r"(a), "r"(ha), "r"(b), "r"(hb), "r"(idesc), "r"(acc));
+                    acc = 1;
+                    a += stepA;
+                    b += 2 * NB;
+                }
+            }
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&bar))
+                     : "memory");
+    }
+    if (tid == 0 && !mbar_wait(smem_u32(&bar), 0)) abort_flag = 1;
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    if (abort_flag) {
+        if (tid == 0 && g.error) atomicExch(g.error, kTimeoutCode);
+    } else {
+        // warp w reads TMEM lanes 32 (w % 4) .. + 31 of every other tile; a lane holds one pixel's NB channels
+        for (int t = warp >> 2; t < tiles; t += 2) {
+            __syncwarp();
+            uint32_t r[NB];
+            const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(t * NB);
+#pragma unroll
+            for (int h = 0; h < NB; h += 16)
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                    "%14, %15}, [%16];"
+                    : "=r"(r[h + 0]), "=r"(r[h + 1]), "=r"(r[h + 2]), "=r"(r[h + 3]), "=r"(r[h + 4]), "=r"(r[h + 5]),
+                      "=r"(r[h + 6]), "=r"(r[h + 7]), "=r"(r[h + 8]), "=r"(r[h + 9]), "=r"(r[h + 10]), "=r"(r[h + 11]),
+                      "=r"(r[h + 12]), "=r"(r[h + 13]), "=r"(r[h + 14]), "=r"(r[h + 15])
+                    : "r"(taddr + (uint32_t)h));
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int e = 0; e < NB; ++e) asm volatile("" : "+r"(r[e]));  // the values exist from here on
+            const int o = t * 128 + (warp & 3) * 32 + lane, y = o / wp, x = o - y * wp;
+            if (y >= rows || x >= g.W) continue;
+            const long long m = (img * g.H + y0 + y) * g.W + x;
+#pragma unroll
+            for (int h = 0; h < NB; h += 8) {
+                if (n0 + h >= g.N) break;  // N is a multiple of 8
+                float v[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    v[e] = __uint_as_float(r[h + e]) + sbias[h + e];
+                    if (g.relu) v[e] = fmaxf(v[e], 0.f);
+                }
+                if (g.out_bf16) store_bf8(g.out_bf16 + m * g.N + n0 + h, v);
+                else store_f8(g.out + m * g.N + n0 + h, v);
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(g.cols));
+}
+
+}  // namespace nn
+}  // namespace octo

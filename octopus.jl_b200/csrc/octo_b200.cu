@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "../../include/octo_b200.h"
+#include "k_conv.cuh"
 #include "k_gauss.cuh"
 #include "k_line.cuh"
 #include "k_moments.cuh"
@@ -253,6 +254,22 @@ void launch_gemm(const GemmArgs &g, int splits, cudaStream_t st) {
     else if (bn == 64) go(k_umma_gemm<64>);
     else if (bn == 128) go(k_umma_gemm<128>);
     else go(k_umma_gemm<256>);
+}
+
+// A 3x3 convolution of B images by bands (k_conv.cuh); false when no band of the image fits a CTA.
+bool launch_conv(ConvArgs g, int B, cudaStream_t st) {
+    ConvArgs wide = g;
+    const double narrow_cost = conv_plan(g, B, 16), wide_cost = g.N <= 16 ? kConvNone : conv_plan(wide, B, 32);
+    if (std::min(narrow_cost, wide_cost) == kConvNone) return false;
+    const int nb = wide_cost <= narrow_cost ? 32 : 16;
+    if (nb == 32) g = wide;
+    const size_t smem = conv_smem(g.C, nb, g.plane);
+    const dim3 grid((unsigned)((g.H + g.R - 1) / g.R), (unsigned)B, (unsigned)((g.N + nb - 1) / nb));
+    void (*kernel)(const ConvArgs) = nb == 16 ? k_conv3<16> : k_conv3<32>;
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    launch_pdl(kernel, grid, kConvThreads, smem, st, g);
+    return true;
 }
 }  // namespace nn
 }  // namespace octo
