@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(256) k_cnn_wgrad_reduce(const float *__restric
         const int terms = bias ? kBiasBlocks : splits;
         float s = 0.f;
         if (i < count) {
-#pragma unroll 4
+#pragma unroll 8
             for (int z = warp; z < terms; z += 8) s += p[z * count + i];
         }
         red[warp][lane] = s;

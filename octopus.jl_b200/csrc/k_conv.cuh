@@ -106,11 +106,15 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3(const __grid_constant__ 
     if (tid < NB) sbias[tid] = g.bias && n0 + tid < g.N ? g.bias[n0 + tid] : 0.f;
     {
         const int k8 = 9 * c8, chunks = g.C == 8 ? 12 : k8;
-        for (int i = tid; i < chunks * NB; i += kConvThreads) {  // an even number of chunks: C = 8 or C % 16 == 0
-            const int pair = i / (2 * NB), r = i - pair * 2 * NB, k = 2 * pair + (r & 1), n = r >> 1;
-            const int src = g.C == 8 ? (k >> 2) * 3 + (k & 3) : k;
-            const bool ok = n0 + n < g.N && (g.C != 8 || (k & 3) < 3);
-            cp_async16(sB + (uint32_t)((k * NB + n) * 16), ok ? g.w + ((long long)(n0 + n) * k8 + src) * 8 : g.w, ok ? 16 : 0);
+        // a thread keeps its channel and its parity of chunk: 2 NB divides the block
+        const int r = tid % (2 * NB), n = r >> 1;
+        constexpr int kStep = kConvThreads / NB;
+        const bool row = n0 + n < g.N;
+        const bf16 *src = g.w + (long long)(row ? n0 + n : 0) * k8 * 8;
+        for (int k = 2 * (tid / (2 * NB)) + (r & 1); k < chunks; k += kStep) {  // chunks is even: C = 8 or C % 16 == 0
+            const int from = g.C == 8 ? (k >> 2) * 3 + (k & 3) : k;
+            const bool ok = row && (g.C != 8 || (k & 3) < 3);
+            cp_async16(sB + (uint32_t)((k * NB + n) * 16), ok ? src + from * 8 : g.w, ok ? 16 : 0);
         }
     }
     pdl_wait();
@@ -124,12 +128,18 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3(const __grid_constant__ 
     }
     // input rows y0 - 1 .. y0 + rows, zero outside the image
     {
-        const int Cs = g.C - g.Cu, count = (rows + 2) * wp * c8;
         // C = 8 multiplies the pixel after the last by the chunk of zeros: it must be finite
         if (g.C == 8 && tid == 0) cp_async16(sA + (uint32_t)((rows + 2) * wp * 16), g.in, 0);
-        for (int i = tid; i < count; i += kConvThreads) {
-            const int p = i / c8, k = i - p * c8, py = p / wp;
-            const int y = y0 - 1 + py, x = p - py * wp - 1, c = k * 8;
+        // One 16-byte chunk of a pixel a step: the chunks of a pixel lie side by side in memory, so neighbouring
+        // threads take them.  Where 256 is a multiple of c8 a thread keeps its chunk and walks the pixels by additions
+        // alone (with a division or two a chunk this loop was the layer's longest part).
+        const int Cs = g.C - g.Cu, pixels = (rows + 2) * wp;
+        const bool walk = kConvThreads % c8 == 0;
+        const int dp = walk ? kConvThreads / c8 : 1, dy = dp / wp, dx = dp - dy * wp;
+        int k = tid % c8, p = walk ? tid / c8 : 0, y = y0 - 1 + p / wp, x = p % wp - 1;
+        if (!walk && tid >= c8) p = pixels;  // c8 threads take every pixel (no network of this library's)
+        for (; p < pixels; p += dp) {
+            const int c = k * 8;
             const uint32_t dst = sA + (uint32_t)((k * g.plane + p) * 16);
             const bool in = y >= 0 && y < g.H && x >= 0 && x < g.W;
             if (g.pool) {
@@ -142,15 +152,21 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3(const __grid_constant__ 
                     for (int e = 0; e < 8; ++e) v[e] = 0.25f * (q0.v[e] + q1.v[e] + q2.v[e] + q3.v[e]);
                 }
                 store_bf8(reinterpret_cast<bf16 *>(g_umma_smem + (dst - sB)), v);
-                continue;
+            } else {
+                const bf16 *s = g.in;
+                if (in) {
+                    if (!g.skip) s = g.in + ((img * g.H + y) * g.W + x) * g.C + c;
+                    else if (c < g.Cu) s = g.in + ((img * (g.H / 2) + y / 2) * (g.W / 2) + x / 2) * g.Cu + c;
+                    else s = g.skip + ((img * g.H + y) * g.W + x) * Cs + (c - g.Cu);
+                }
+                cp_async16(dst, s, in ? 16 : 0);
             }
-            const bf16 *s = g.in;
-            if (in) {
-                if (!g.skip) s = g.in + ((img * g.H + y) * g.W + x) * g.C + c;
-                else if (c < g.Cu) s = g.in + ((img * (g.H / 2) + y / 2) * (g.W / 2) + x / 2) * g.Cu + c;
-                else s = g.skip + ((img * g.H + y) * g.W + x) * Cs + (c - g.Cu);
+            y += dy;
+            x += dx;
+            if (x >= wp - 1) {
+                x -= wp;
+                ++y;
             }
-            cp_async16(dst, s, in ? 16 : 0);
         }
     }
     cp_async_commit();
