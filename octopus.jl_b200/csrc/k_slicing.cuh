@@ -126,30 +126,18 @@ __global__ void __launch_bounds__(kLaneFoldThreads, 1) k_lane_fold(const SliceAr
     if (t < 32) lane_sum[lane0 + t] = s;
 }
 
-// In-order sum of n shared-memory values (the order of a plain loop): a chain of dependent additions, so the next
-// sixteen values are loaded while the current sixteen are added.  A collide runs three of these chains one after the
-// other; with loads and additions in turn they were 77 us of a small collide's 395.
+// In-order sum of n shared-memory values, sixteen loads ahead of the adds (the order of a plain loop).  A collide runs
+// three of these chains one after the other, 4096 dependent additions each: 77 us, at the addition's latency (loading
+// the next sixteen during the adds measured 2 us a chain slower).
 __device__ __forceinline__ double serial_sum(const double *v, int n) {
-    auto load = [&](double (&w)[16], int t) {
+    double s = 0.0;
+    int t = 0;
+    for (; t + 16 <= n; t += 16) {
+        double w[16];
 #pragma unroll
         for (int u = 0; u < 16; ++u) w[u] = v[t + u];
-    };
-    double s = 0.0, a[16], b[16];
-    auto add = [&](const double (&w)[16]) {
 #pragma unroll
         for (int u = 0; u < 16; ++u) s += w[u];
-    };
-    int t = 0;
-    if (n >= 16) load(a, 0);
-    for (; t + 32 <= n; t += 32) {
-        load(b, t + 16);
-        add(a);
-        if (t + 48 <= n) load(a, t + 32);
-        add(b);
-    }
-    if (t + 16 <= n) {
-        add(a);
-        t += 16;
     }
     for (; t < n; ++t) s += v[t];
     return s;
