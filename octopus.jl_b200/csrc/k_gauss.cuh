@@ -137,15 +137,28 @@ __global__ void __launch_bounds__(kGaussThreads) k_gauss_sums(GaussArgs A) {
     const R *c[4] = {gcol<R>(A, S.beam, 0), gcol<R>(A, S.beam, 1), gcol<R>(A, S.beam, 2), gcol<R>(A, S.beam, 3)};
     const double x0 = c[0][S.start], px0 = c[1][S.start], y0 = c[2][S.start], py0 = c[3][S.start];
     double s[kGaussSums] = {};
+    // four particles' loads in flight before the first is summed
+    constexpr int kAhead = 4;
     const long long end = min(S.n, (long long)bm.y + kGaussChunk);
-    for (long long k = bm.y + threadIdx.x; k < end; k += kGaussThreads) {
-        const long long i = S.start + k;
-        const double dx = (double)c[0][i] - x0, dpx = (double)c[1][i] - px0, dy = (double)c[2][i] - y0,
-                     dpy = (double)c[3][i] - py0;
-        s[0] += dx; s[1] += dpx; s[2] += dy; s[3] += dpy;
-        s[4] += dx * dx; s[5] += dpx * dpx; s[6] += dy * dy; s[7] += dpy * dpy;
-        s[8] += dx * dpx; s[9] += dy * dpy;
-        if (A.coupled) { s[10] += dx * dy; s[11] += dx * dpy; s[12] += dpx * dy; s[13] += dpx * dpy; }
+    for (long long k0 = bm.y + threadIdx.x; k0 < end; k0 += kAhead * kGaussThreads) {
+        R v[kAhead][4];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const long long i = S.start + k0 + u * kGaussThreads;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (k0 + u * kGaussThreads < end) v[u][q] = c[q][i];
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            if (k0 + u * kGaussThreads >= end) break;
+            const double dx = (double)v[u][0] - x0, dpx = (double)v[u][1] - px0, dy = (double)v[u][2] - y0,
+                         dpy = (double)v[u][3] - py0;
+            s[0] += dx; s[1] += dpx; s[2] += dy; s[3] += dpy;
+            s[4] += dx * dx; s[5] += dpx * dpx; s[6] += dy * dy; s[7] += dpy * dpy;
+            s[8] += dx * dpx; s[9] += dy * dpy;
+            if (A.coupled) { s[10] += dx * dy; s[11] += dx * dpy; s[12] += dpx * dy; s[13] += dpx * dpy; }
+        }
     }
     __shared__ double red[kGaussSums][kGaussThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -313,7 +326,8 @@ __global__ void __launch_bounds__(kGaussThreads, kGaussKickBlocks) k_gauss_kick(
 }
 
 // Pair luminosity (gaussian.jl:64-108): sum of density * 2 pi over the sampled slice / 2 pi * klum.  One warp per
-// sampling task: each lane takes every 32nd of its kick blocks' partials, then the lanes are folded pairwise.
+// sampling task: each lane takes every 32nd of its kick blocks' partials, then the lanes are folded pairwise.  One
+// launch after the last front folds them all (a launch a front lay on the chain of fronts, 6 us each).
 __global__ void __launch_bounds__(32) k_gauss_lum(GaussArgs A, const int *lum_task, const int *first, const int *count) {
     pdl_wait();
     pdl_release();

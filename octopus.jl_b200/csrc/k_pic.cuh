@@ -358,6 +358,7 @@ __global__ void __launch_bounds__(256) k_hyb_moments(Collide C, int task0) {
     const bool gate = isfinite(C.o.coupling_tol);  // the cross-plane sums only when the coupled path can read them
     if (n > 0) {
         const double x0 = X[0], px0 = PX[0], y0 = Y[0], py0 = PY[0];
+#pragma unroll 4
         for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
             const double dx = (double)X[k] - x0, dpx = (double)PX[k] - px0, dy = (double)Y[k] - y0, dpy = (double)PY[k] - py0;
             a[0] += dx; a[1] += dpx; a[2] += dy; a[3] += dpy;

@@ -1862,7 +1862,7 @@ void CollideJob::run_gaussian(const SliceInfo &S1, const SliceInfo &S2) {
             launches += (F.nsb ? 1 : 0) + 1;
         }
         {
-            PhaseScope ps(c, OCTO_PHASE_KICK, st, 2);
+            PhaseScope ps(c, OCTO_PHASE_KICK, st, 1);
             GaussArgs Ak = A;
             Ak.blockmap = c->g_bmap.p + smap.size() + F.kb0;
             Ak.lum_partial = c->g_lum_partial.p + F.kb0;
@@ -1871,10 +1871,13 @@ void CollideJob::run_gaussian(const SliceInfo &S1, const SliceInfo &S2) {
                 if (F.nkb && A.coupled) launch_pdl(k_gauss_kick<decltype(r), true>, F.nkb, kGaussThreads, 0, st, Ak);
                 else if (F.nkb) launch_pdl(k_gauss_kick<decltype(r), false>, F.nkb, kGaussThreads, 0, st, Ak);
             });
-            // the fold reads the kick partials by their index over all fronts (lfirst)
-            if (F.nl) launch_pdl(k_gauss_lum, F.nl, 32, 0, st, A, d_ltask + F.l0, d_lfirst + F.l0, d_lcount + F.l0);
-            launches += (F.nkb ? 1 : 0) + (F.nl ? 1 : 0);
+            launches += F.nkb ? 1 : 0;
         }
+    }
+    if (!ltask.empty()) {  // the kick partials carry their index over all fronts (lfirst)
+        PhaseScope ps(c, OCTO_PHASE_KICK, st, 1);
+        launch_pdl(k_gauss_lum, (int)ltask.size(), 32, 0, st, A, d_ltask, d_lfirst, d_lcount);
+        ++launches;
     }
     CK(cudaGetLastError());
 }
