@@ -973,16 +973,19 @@ __device__ __forceinline__ Q quantize(R x) {
 }
 template <class R, int METHOD, bool TOTAL = false, bool ROT = false, class Q = long long>
 __device__ __forceinline__ long long deposit_taps(R u, R v, int nw, int nh, R scale, Q *grid, int ld, int rot = 0) {
-    constexpr int NT = METHOD == 0 ? 2 : 3;
-    int ix, iy;
     long long total = 0;
-    R wx[NT], wy[NT];
-    if (METHOD == 0) { cic_weights(u, nw, ix, wx); cic_weights(v, nh, iy, wy); }
-    else { tsc_weights(u, nw, ix, wx); tsc_weights(v, nh, iy, wy); }
-    const int c0 = (iy - 1) * ld + (ix - 1);
     if constexpr (METHOD == 0) {
-        Q q0 = quantize<Q>(wx[0] * wy[0] * scale), q1 = quantize<Q>(wx[0] * wy[1] * scale);
-        Q q2 = quantize<Q>(wx[1] * wy[0] * scale), q3 = quantize<Q>(wx[1] * wy[1] * scale);
+        // a particle outside the mesh has no charge on it; the scale is a power of two, so scaling one factor rounds as
+        // scaling the product
+        if (!cic_inside(u, v, nw, nh)) return 0;
+        int bx, by;
+        R fx, fy;
+        cic_axis(u, nw, bx, fx);
+        cic_axis(v, nh, by, fy);
+        const int c0 = by * ld + bx;
+        const R gy = R(1) - fy, sx = fx * scale, sg = (R(1) - fx) * scale;
+        Q q0 = quantize<Q>(sg * gy), q1 = quantize<Q>(sg * fy);
+        Q q2 = quantize<Q>(sx * gy), q3 = quantize<Q>(sx * fy);
         if (TOTAL) total = (long long)q0 + q1 + q2 + q3;
         int o0 = c0, o1 = c0 + ld, o2 = c0 + 1, o3 = c0 + ld + 1;
         if constexpr (ROT) {  // a separate instantiation: the permutation costs the unrotated deposit nothing
@@ -1000,6 +1003,12 @@ __device__ __forceinline__ long long deposit_taps(R u, R v, int nw, int nh, R sc
         atom_add(&grid[o2], q2);
         atom_add(&grid[o3], q3);
     } else {
+        constexpr int NT = 3;
+        int ix, iy;
+        R wx[NT], wy[NT];
+        tsc_weights(u, nw, ix, wx);
+        tsc_weights(v, nh, iy, wy);
+        const int c0 = (iy - 1) * ld + (ix - 1);
 #pragma unroll
         for (int m = 0; m < NT; ++m)
 #pragma unroll
@@ -1113,11 +1122,11 @@ __global__ void __launch_bounds__(1024, 1) k_deposit(Collide C, int plane0) {
             }
             const R xd = cx + cpx * s;
             const R yd = cy + cpy * s;
-            if (count_dropped && !(isfinite(xd) && xlo <= xd && xd <= xhi && isfinite(yd) && ylo <= yd && yd <= yhi))
+            if (count_dropped && !(xlo <= xd && xd <= xhi && ylo <= yd && yd <= yhi))
                 ++outside;
             else if (count_dropped == 2) {  // :sigma and :source_slice: the particle at the other boundary too
                 const R x2 = cx + cpx * s2, y2 = cy + cpy * s2;
-                if (!(isfinite(x2) && xlo <= x2 && x2 <= xhi && isfinite(y2) && ylo <= y2 && y2 <= yhi)) ++outside;
+                if (!(xlo <= x2 && x2 <= xhi && ylo <= y2 && y2 <= yhi)) ++outside;
             }
             total += deposit_taps<R, METHOD, TOT, ROT, QA>((xd - x0) * hxi, (yd - y0) * hyi, nx, ny, scale, acc, nx, rot);
             cx = nx_; cpx = npx; cy = ny_; cpy = npy;
@@ -1196,14 +1205,14 @@ __global__ void __launch_bounds__(1024, 1) k_deposit_node3(Collide C, int plane0
         const R xl = cx + cpx * sL, yl = cy + cpy * sL;
         const R xr = cx + cpx * sR, yr = cy + cpy * sR;
         if (okL) {
-            if (!(isfinite(xl) && xL0 <= xl && xl <= xLhi && isfinite(yl) && yL0 <= yl && yl <= yLhi)) ++outside;
+            if (!(xL0 <= xl && xl <= xLhi && yL0 <= yl && yl <= yLhi)) ++outside;
             deposit_taps<R, METHOD, false, false, int>((xl - xL0) * hxiL, (yl - yL0) * hyiL, nx, ny, scale, sq, nx);
             if (z)
                 deposit_taps<R, METHOD, false, false, int>((xr - xL0) * hxiL, (yr - yL0) * hyiL, nx, ny, scale, sq + 2 * cells,
                                                            nx);
         }
         if (okR) {
-            if (!(isfinite(xr) && xR0 <= xr && xr <= xRhi && isfinite(yr) && yR0 <= yr && yr <= yRhi)) ++outside;
+            if (!(xR0 <= xr && xr <= xRhi && yR0 <= yr && yr <= yRhi)) ++outside;
             deposit_taps<R, METHOD, false, false, int>((xr - xR0) * hxiR, (yr - yR0) * hyiR, nx, ny, scale, sq + cells, nx);
         }
         cx = nx_; cpx = npx; cy = ny_; cpy = npy;
@@ -2031,21 +2040,40 @@ template <class R, int METHOD>
 struct Taps {
     static constexpr int NT = METHOD == 0 ? 2 : 3;
     int c0;          // first cell (x-outer, y-inner order follows from c0 + m + k*nx)
+    bool inside;
     R w[NT * NT];
     // hxi, hyi: reciprocals of the mesh spacing g.w/(nx-1), g.h/(ny-1), computed once per block.  The
     // reference divides by the spacing (pic_cpu.jl:2601-2602); in FP64 the product differs from that
     // quotient by at most 1.5 ulp of u, a ~1e-14 relative change of the interpolation weights.
     __device__ __forceinline__ Taps(const DevOptions &o, const GridR<R> &g, R hxi, R hyi, R x, R y) {
         const R u = (x - g.x0) * hxi, v = (y - g.y0) * hyi;
-        int ix, iy; R wx[NT], wy[NT];
-        if (METHOD == 0) { cic_weights(u, o.nx, ix, wx); cic_weights(v, o.ny, iy, wy); }
-        else { tsc_weights(u, o.nx, ix, wx); tsc_weights(v, o.ny, iy, wy); }
-        c0 = (iy - 1) * o.nx + (ix - 1);
+        if constexpr (METHOD == 0) {
+            inside = cic_inside(u, v, o.nx, o.ny);
+            int bx, by;
+            R fx, fy;
+            cic_axis(u, o.nx, bx, fx);
+            cic_axis(v, o.ny, by, fy);
+            const R gx = R(1) - fx, gy = R(1) - fy;
+            c0 = by * o.nx + bx;
+            w[0] = gx * gy;
+            w[1] = gx * fy;
+            w[2] = fx * gy;
+            w[3] = fx * fy;
+        } else {
+            inside = true;
+            int ix, iy;
+            R wx[NT], wy[NT];
+            tsc_weights(u, o.nx, ix, wx);
+            tsc_weights(v, o.ny, iy, wy);
+            c0 = (iy - 1) * o.nx + (ix - 1);
 #pragma unroll
-        for (int m = 0; m < NT; ++m)
+            for (int m = 0; m < NT; ++m)
 #pragma unroll
-            for (int k = 0; k < NT; ++k) w[m * NT + k] = wx[m] * wy[k];
+                for (int k = 0; k < NT; ++k) w[m * NT + k] = wx[m] * wy[k];
+        }
     }
+    // a sum over the taps: nothing for a particle outside the mesh (its taps are some cell's, TSC's have zero weights)
+    __device__ __forceinline__ R in(R sum) const { return METHOD != 0 || inside ? sum : R(0); }
     __device__ __forceinline__ int cell(int t, int nx) const { return c0 + (t / NT) + (t % NT) * nx; }
 };
 
@@ -2059,6 +2087,7 @@ template <class R>
 struct KickJob {
     GridR<R> gL, gR;
     R hxL, hyL, hxR, hyR;  // reciprocal spacings
+    R xhi, yhi;            // gL's upper ends
     R c_src, hzi, zbias, ks;
     long long fld_start, fld_n, plane_off;
     int fld_beam, ok;
@@ -2127,7 +2156,7 @@ __device__ __forceinline__ void kick_particle(const Collide &C, const KickJob<R>
         // single-plane interpolations reduce exactly to w * E (pic_cpu.jl:1517-1528).
         const GridR<R> &gL = J.gL, &gR = J.gR;
         const FC *FL = base, *FR = base + CV * pc;  // the L plane's w word holds phi_Z (k_conv_field)
-        if (!(isfinite(x) && gL.x0 <= x && x <= gL.x0 + gL.w && isfinite(y) && gL.y0 <= y && y <= gL.y0 + gL.h))
+        if (!(gL.x0 <= x && x <= J.xhi && gL.y0 <= y && y <= J.yhi))  // (a finite mesh: no NaN or infinity passes)
             atomicAdd((unsigned long long *)&C.status->dropped, 1ull);
         R KxL = 0, KyL = 0, Kz = 0, KxR = 0, KyR = 0;
         {
@@ -2141,6 +2170,9 @@ __device__ __forceinline__ void kick_particle(const Collide &C, const KickJob<R>
                 if (kPrecision) Kz += tp.w[t] * phz;  // the Z plane holds phi_L - phi_Z
                 else Kz += tp.w[t] * (phl - phz);
             }
+            KxL = tp.in(KxL);
+            KyL = tp.in(KyL);
+            Kz = tp.in(Kz);
         }
         {
             const Taps<R, METHOD> tp(o, gR, J.hxR, J.hyR, x, y);
@@ -2163,6 +2195,8 @@ __device__ __forceinline__ void kick_particle(const Collide &C, const KickJob<R>
                     KyR += tp.w[t] * ey;
                 }
             }
+            KxR = tp.in(KxR);
+            KyR = tp.in(KyR);
         }
         px += ks * (zL * KxL + zR * KxR);
         py += ks * (zL * KyL + zR * KyR);
@@ -2192,6 +2226,9 @@ __device__ __forceinline__ void kick_particle(const Collide &C, const KickJob<R>
                 Kz += tp.w[q] * (bL * pl + bM * pm + bR * pr);
             }
         }
+        Kx = tp.in(Kx);
+        Ky = tp.in(Ky);
+        Kz = tp.in(Kz);
         px += ks * Kx;
         py += ks * Ky;
         if (lk) { if (kPrecision) dpz += ks * Kz * J.hzi; else pz += ks * Kz * J.hzi; }
@@ -2215,6 +2252,9 @@ __device__ __forceinline__ void kick_particle(const Collide &C, const KickJob<R>
                 Kz += tp.w[q] * (pl - pr);
             }
         }
+        Kx = tp.in(Kx);
+        Ky = tp.in(Ky);
+        Kz = tp.in(Kz);
         if (HYB && J.hyb == 2) {
             // Rotated add-back of the tilted Gaussian through _cp_covariance_kick at both boundaries, blended in z
             // (gaussian_pic.jl:837-854)
@@ -2322,6 +2362,8 @@ __global__ void __launch_bounds__(kKickThreads, sizeof(R) == 8 ? 2 : 4)
         }
         J.gL = grid_r<R>(gL);
         J.gR = grid_r<R>(gR);
+        J.xhi = J.gL.x0 + J.gL.w;
+        J.yhi = J.gL.y0 + J.gL.h;
         J.hxL = (R)(1.0 / (gL.w / (double)(C.o.nx - 1))); J.hyL = (R)(1.0 / (gL.h / (double)(C.o.ny - 1)));
         J.hxR = (R)(1.0 / (gR.w / (double)(C.o.nx - 1))); J.hyR = (R)(1.0 / (gR.h / (double)(C.o.ny - 1)));
         J.c_src = (R)T.c_src; J.hzi = (R)T.hzi; J.zbias = (R)T.zbias; J.ks = (R)T.ks;
