@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(1024) k_fold_stats(const SliceArgs<R> A, int s
     }
     __syncthreads();
     if (threadIdx.x != 0) return;
-    const double s = serial_sum(sl, (int)min((long long)kFoldLanes, n));  // lanes past n hold zeros
+    const double s = n >= kFoldLanes ? serial_sum(sl, kFoldLanes) : serial_sum(sl, (int)n);  // lanes past n hold zeros
     if (stage == 0) {
         double lo = INFINITY, hi = -INFINITY;
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { lo = jmin(lo, rlo[w]); hi = jmax(hi, rhi[w]); }
@@ -681,7 +681,8 @@ __global__ void __launch_bounds__(1024) k_slice_finish(const SliceArgs<R> A) {
     info->weight[s] = (double)cnt / (double)n;
     const double *b = info->boundary;
     if (fold) {
-        info->center[s] = serial_sum(sl, (int)min((long long)kFoldLanes, cnt)) / (double)cnt;  // the others hold zeros
+        const double sum = cnt >= kFoldLanes ? serial_sum(sl, kFoldLanes) : serial_sum(sl, (int)cnt);  // the others hold zeros
+        info->center[s] = sum / (double)cnt;
     } else {
         info->center[s] = (b[s] + b[s + 1]) / 2;
     }
