@@ -271,11 +271,16 @@ struct Cnn {
         const long long M = ml(L.level, B), ld = round8(M);
         const int hh = hl(L.level), ww = wl(L.level);
         im2col_t<1>((const bf16 *)g.p, gt.p, M, hh, ww, L.cout, ld, st);
-        im2col_t<9>(in, colt.p, M, hh, ww, L.cin, ld, st);
+        // where 8 pixels lie in one row the GEMM takes its nine taps from three column shifts (a third of the writes,
+        // and reads that L2 holds); else from the whole transposed im2col
+        const bool shifts = ww % 8 == 0;
+        if (shifts) im2col_t<3>(in, colt.p, M, hh, ww, L.cin, ld, st);
+        else im2col_t<9>(in, colt.p, M, hh, ww, L.cin, ld, st);
         const int splits = wgrad_splits(l, B);
         GemmArgs a{};
         a.M = 9 * L.cin; a.N = L.cout; a.K = (int)ld;
-        a.A = colt.p; a.lda = ld; a.a_mode = 0;
+        a.A = colt.p; a.lda = ld; a.a_mode = shifts ? 3 : 0;
+        a.H = hh; a.W = ww; a.C = L.cin;
         a.B = gt.p; a.ldb = ld;
         a.out = part.p; a.ldc = L.cout; a.split_stride = (long long)a.M * L.cout;
         const long long chunks = (ld + kBK - 1) / kBK;

@@ -148,11 +148,12 @@ __global__ void k_cnn_pool_adj_add(const float *__restrict__ dp, float *__restri
 }
 
 // Transposed im2col of a 3x3 / pad-1 convolution's NHWC input: out[(tap * C + c)][m] = x[pixel m shifted by tap][c]
-// (zero outside the image and for M <= m < ld); TAPS = 1: the plain transpose, out[c][m] = x[m][c].
+// (zero outside the image and for M <= m < ld); TAPS = 1: the plain transpose, out[c][m] = x[m][c]; TAPS = 3: the three
+// column shifts alone, out[(dx * C + c)][m] = x[pixel m shifted by dx - 1 in its row][c].
 // Bound by the write of out.  A block moves CG channels of 2048 / CG pixels for one tap through shared memory: one
 // 16-byte load of 8 channels and one 16-byte store of 8 pixels a thread (one element a thread, with its own divisions
 // and a load 2 C bytes from its neighbour's, took 1.79 ms of a batch-64 training step; this takes
-// 0.23 ms, for all layers).
+// 0.23 ms, for all layers, and 0.12 ms with the column shifts alone where the weight gradient's GEMM can take them).
 // grid (ceil(ld / pixels), C / CG, TAPS); out rows and ld are multiples of 8 elements.
 constexpr int kIm2colThreads = 256;
 template <int CG, int TAPS>
@@ -173,7 +174,7 @@ __global__ void __launch_bounds__(kIm2colThreads) k_cnn_im2col_t(const bf16 *__r
                 v = *reinterpret_cast<const uint4 *>(x + m * C + c0 + q * 8);
             } else {
                 const long long row = m / W;
-                const int xx = (int)(m - row * W) + tap % 3 - 1, dy = tap / 3 - 1, yy = (int)(row % H) + dy;
+                const int xx = (int)(m - row * W) + tap % 3 - 1, dy = TAPS == 3 ? 0 : tap / 3 - 1, yy = (int)(row % H) + dy;
                 if (yy >= 0 && yy < H && xx >= 0 && xx < W)
                     v = *reinterpret_cast<const uint4 *>(x + (m + (long long)dy * W + tap % 3 - 1) * C + c0 + q * 8);
             }

@@ -1,5 +1,5 @@
-// BF16 GEMM on the fifth-generation tensor cores (tcgen05 / UMMA), the contraction behind the learned
-// field correction's convolutions (forward, input gradient, weight gradient).
+// BF16 GEMM on the fifth-generation tensor cores (tcgen05 / UMMA): the weight gradients of the learned field
+// correction's convolutions, and the convolutions themselves where an image is too wide for k_conv.cuh's bands.
 //
 //   C[M, N] (fp32) = sum_k A[m, k] * B[n, k]            (both operands K-major)
 //
@@ -40,7 +40,10 @@ struct GemmArgs {
     const __nv_bfloat16 *A;       // a_mode 0: A[m * lda + k]
     long long lda;
     int a_mode;                   // 0 dense, 1 implicit 3x3 / pad-1 convolution of an NHWC tensor, 2 the same
-                                  // of [nearest-upsampled A, A2] concatenated along channels (a U-Net decoder)
+                                  // of [nearest-upsampled A, A2] concatenated along channels (a U-Net decoder),
+                                  // 3 the transposed im2col (rows 9 C, K = pixels) from its three column shifts:
+                                  // A(tap C + c, k) = A[((tap % 3) C + c) lda + k + (tap / 3 - 1) W] inside the image
+                                  // (W a multiple of 8, so that 8 pixels lie in one row; K the pixel count)
     int H, W, C;                  // a_mode 1, 2: input height, width, channels (C a multiple of 8); K = 9 C
     const __nv_bfloat16 *A2;      // a_mode 2: the skip tensor [b][H][W][C - Cu]; A is [b][H/2][W/2][Cu]
     int Cu;                       // a_mode 2: channels from the upsampled tensor (a multiple of 8)
@@ -182,6 +185,10 @@ __global__ void __launch_bounds__(kGemmThreads, 2) k_umma_gemm(const GemmArgs g)
                 if (g.a_mode == 0) {
                     ry[it] = 0;
                     rbase[it] = (long long)m * g.lda;
+                } else if (g.a_mode == 3) {  // ry: the tap's row shift plus one
+                    const int tap = m / g.C;
+                    ry[it] = tap / 3;
+                    rbase[it] = ((long long)(tap % 3) * g.C + (m - tap * g.C)) * g.lda + (long long)(tap / 3 - 1) * g.W;
                 } else {
                     const int b = div_small(m, hw, inv_hw), rem = m - b * hw;
                     const int y = div_small(rem, g.W, inv_w), x = rem - y * g.W;
@@ -193,8 +200,10 @@ __global__ void __launch_bounds__(kGemmThreads, 2) k_umma_gemm(const GemmArgs g)
         // loads of K chunk i into stage s (every thread: its A rows, then its share of B)
         auto load_stage = [&](int i, int s) {
             const int k = kb + i * kBK + kc_t * 8;
-            int dy = 0, dx = 0, c = k;
-            if (g.a_mode != 0) {  // both convolution modes: tap (ky, kx) and channel of k
+            int dy = 0, dx = 0, c = k, yk = 0;
+            if (g.a_mode == 3) {
+                yk = k / g.W % g.H;  // the image row of these 8 pixels
+            } else if (g.a_mode != 0) {  // both convolution modes: tap (ky, kx) and channel of k
                 const int tap = k / g.C;
                 c = k - tap * g.C;
                 dy = tap / 3 - 1;
@@ -210,6 +219,11 @@ __global__ void __launch_bounds__(kGemmThreads, 2) k_umma_gemm(const GemmArgs g)
                     if (g.a_mode == 0) {
                         src = g.A + rbase[it] + k;
                         bytes = 16;
+                    } else if (g.a_mode == 3) {
+                        if ((unsigned)(yk + ry[it] - 1) < (unsigned)g.H) {
+                            src = g.A + rbase[it] + k;
+                            bytes = 16;
+                        }
                     } else {
                         const int yy = ry[it] + dy, xx = rx[it] + dx;
                         if (yy >= 0 && yy < g.H && xx >= 0 && xx < g.W) {
