@@ -702,8 +702,8 @@ def time_soft_gaussian(ob, e0, p0, me, mp, rt, local_rank, args, stream, cpu_sid
 
 
 def time_observer(ob, e0, p0, args, stream):
-    """The moment observer on both beams (the default orders 1:2, 27 moments): each observation is two passes
-    over the beam (means, then the 21 second-order sums) whose row stays on the device; 96 bytes per
+    """The moment observer on both beams (the default orders 1:2, 27 moments): each observation is one pass
+    over the beam (the sums and the 21 products about a pivot) whose row stays on the device; 48 bytes per
     particle read."""
     import torch
     beams = {"electron": ob.Beam(e0.clone(), ob.BeamParams(-1.0, ob.EMASS_EV, 10e9, 0.0, 1.7e11)),
@@ -730,7 +730,7 @@ def time_observer(ob, e0, p0, args, stream):
         ev1.record(stream)
         torch.cuda.synchronize()
         ms = ev0.elapsed_time(ev1) / K
-        gbs = beams[b].n * 96 / (ms / 1e3) / 1e9
+        gbs = beams[b].n * 48 / (ms / 1e3) / 1e9
         out[b] = {"us_per_row": ms * 1e3, "achieved_gbs": gbs, "frac_of_hbm": gbs / hbm}
     out["note"] = ("rows are written to a device record buffer; the host reads them once per flush, so "
                    "observing a turn adds no host synchronisation")

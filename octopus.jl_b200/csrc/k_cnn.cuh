@@ -1,5 +1,5 @@
 // Element-wise and reduction kernels of the learned field correction's CNN (a 4-level U-Net of 3x3
-// convolutions, 32 base channels).  The convolutions themselves are tensor-core GEMMs (k_umma.cuh); these
+// convolutions, 32 base channels).  The convolutions themselves run on the tensor cores (k_conv.cuh, k_umma.cuh); these
 // kernels move activations between them: 2x2 average pooling, nearest upsampling with skip concatenation,
 // the adjoints of both, ReLU masks, transposes and im2col for the weight gradients, the fixed-order
 // reductions of the weight and bias gradients, the loss, and Adam.  Activations are NHWC bf16 with rows

@@ -1738,11 +1738,11 @@ void CollideJob::run_gaussian(const SliceInfo &S1, const SliceInfo &S2) {
     std::vector<int2> smap, kmap;             // sums blocks, kick blocks
     std::vector<int> sfirst, scount;          // per slice: its sums blocks
     std::vector<int> ltask, lfirst, lcount;   // per sampling task: its kick blocks
-    struct Front { int s0, ns, sb0, nsb, t0, nt, kb0, nkb, l0, nl, chunk; };
+    struct Front { int s0, ns, sb0, nsb, t0, nt, kb0, nkb, chunk; };
     std::vector<Front> fronts;
     tasks.clear();
     for (size_t f = 0; f < batches.size(); ++f) {
-        Front F{(int)gs.size(), 0, (int)smap.size(), 0, (int)gt.size(), 0, (int)kmap.size(), 0, (int)ltask.size(), 0, 0};
+        Front F{(int)gs.size(), 0, (int)smap.size(), 0, (int)gt.size(), 0, (int)kmap.size(), 0, 0};
         long long front_n = 0;
         for (const OrderEntry &pr : batches[f]) front_n += S1.count[pr.i - 1] + S2.count[pr.j - 1];
         F.chunk = gauss_kick_chunk(front_n, c->num_sms);
@@ -1791,7 +1791,6 @@ void CollideJob::run_gaussian(const SliceInfo &S1, const SliceInfo &S2) {
         F.nsb = (int)smap.size() - F.sb0;
         F.nt = (int)gt.size() - F.t0;
         F.nkb = (int)kmap.size() - F.kb0;
-        F.nl = (int)ltask.size() - F.l0;
         if (F.ns) fronts.push_back(F);
     }
     ntasks = (int)tasks.size();
