@@ -14,7 +14,7 @@
 //   skip: the input is [nearest-upsampled in (Cu channels), skip] (a decoder level).
 // Bound by latency: a layer is a few microseconds of loads, instructions and stores between two launches.  The im2col
 // GEMM (k_umma.cuh) reads every input nine times in K chunks that wait for one another: a forward pass over 20 planes of
-// 48 x 48 took 304 us with it (split-K folds and pools included) and takes 172 us; a batch-64 training step 2.01 and 1.57 ms.
+// 48 x 48 took 304 us with it (split-K folds and pools included) and takes 160 us; a batch-64 training step 2.01 ms with it, 1.57 ms with the first form of this kernel.
 //
 // The mbarrier wait is bounded (about one second of the global timer); on expiry the kernel records OCTO_ERR_TIMEOUT
 // in *error, frees its TMEM and returns.
@@ -50,8 +50,11 @@ inline size_t conv_smem(int C, int nb, int plane) {
 }
 
 // Rows a band for B images at nb channels a CTA: the least of a launch's fixed latency per wave, the bytes each SM brings
-// in and the instructions it issues, over the bands that fit (half of TMEM, so that two CTAs share an SM, and 200 KB).
-// Returns that cost (about a microsecond a unit), 1e30 when none fits (very wide images: the im2col GEMM runs those).
+// in and the instructions it issues, over the bands that fit (half of TMEM, so that two CTAs share an SM, and kConvSmem:
+// 227 KB less the 1 KB of this kernel itself).  Returns that cost (about a microsecond a unit), 1e30 when none fits (very
+// wide images: the im2col GEMM runs those).  While bands were held to 200 KB the widest decoder layer (256 to 64
+// channels, 12 x 12, 20 images) ran 240 CTAs in two waves, 31 us; now one band an image, 80 CTAs, 19 us.
+constexpr size_t kConvSmem = 226 * 1024;
 constexpr double kConvNone = 1e30;
 inline double conv_plan(ConvArgs &g, int B, int nb) {
     if (g.C % 16 && g.C != 8) return kConvNone;
@@ -62,11 +65,11 @@ inline double conv_plan(ConvArgs &g, int B, int nb) {
         if (tiles * nb > 256) break;
         const int plane = (tiles * 128 + 2 * wp + 4) | 1;
         const size_t smem = conv_smem(g.C, nb, plane);
-        if (smem > 200 * 1024) break;
+        if (smem > kConvSmem) break;
         int cols = 32;
         while (cols < tiles * nb) cols *= 2;
         const long long ctas = (long long)((g.H + R - 1) / R) * B * nblk;
-        const int res = (int)std::min<long long>({(long long)(225 * 1024 / (smem + 1024)), 512 / cols, 8});
+        const int res = (int)std::min<long long>({(long long)(228 * 1024 / (smem + 2048)), 512 / cols, 8});
         const double per_sm = (double)((ctas + 147) / 148), waves = (double)((ctas + 148LL * res - 1) / (148LL * res));
         const double cost = 4.0 * waves + per_sm * (smem * 8.3e-6 + 0.008 * tiles * steps * (nb / 16));
         if (cost < best) {

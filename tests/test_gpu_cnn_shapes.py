@@ -36,3 +36,19 @@ def test_gradients_at_odd_sizes(B, H, W, masked):
             assert np.linalg.norm(a - b) <= 2e-2 * np.linalg.norm(b), (k, np.linalg.norm(a - b) / np.linalg.norm(b))
         off += n + cout
     net.close()
+
+
+@pytest.mark.parametrize("B,H,W", [(20, 48, 48), (64, 32, 32), (64, 16, 16), (3, 16, 64)])
+def test_forward_of_bands_that_fill_shared_memory(B, H, W):
+    """Batches at which the widest decoder layer takes bands of up to 226 KB (one CTA an SM), and small ones."""
+    from oracle import cnn_oracle as co
+    from octo_b200.learned import FieldCorrectionNet
+    net = FieldCorrectionNet(H, W, max_batch=B, seed=11)
+    p = net.get_params()
+    p = p + (0.01 * np.random.default_rng(3).standard_normal(p.size)).astype(np.float32)
+    net.set_params(p)
+    xb, _, _ = _inputs(B, H, W, 5)
+    out = net.forward(xb).cpu().numpy()
+    ref = co.Net(p.astype(np.float64), rounding=True).forward(xb.float().cpu().numpy().astype(np.float64))[..., :2]
+    assert np.linalg.norm(out - ref) <= 1e-2 * np.linalg.norm(ref)  # the bound of test_gpu_cnn.py
+    net.close()
