@@ -14,7 +14,8 @@
 //   skip: the input is [nearest-upsampled in (Cu channels), skip] (a decoder level).
 // Bound by latency: a layer is a few microseconds of loads, instructions and stores between two launches.  The im2col
 // GEMM (k_umma.cuh) reads every input nine times in K chunks that wait for one another: a forward pass over 20 planes of
-// 48 x 48 took 304 us with it (split-K folds and pools included) and takes 160 us; a batch-64 training step 2.01 ms with it, 1.57 ms with the first form of this kernel.
+// 48 x 48 took 304 us with it (split-K folds and pools included) and takes 160 us; a
+// batch-64 training step took 2.01 ms with it, 1.57 ms with the first form of this kernel.
 //
 // The mbarrier wait is bounded (about one second of the global timer); on expiry the kernel records OCTO_ERR_TIMEOUT
 // in *error, frees its TMEM and returns.
