@@ -9,7 +9,9 @@
 // The weights of the CTA's NB output channels lie beside it in the same form.  Warp t's first lane issues every
 // tcgen05.mma (M = 128 pixels, N = NB, K = 16) of tile t into TMEM and commits once; an instruction's operands are two
 // additions away from the one before (rebuilt descriptors made the issuing lane the layer's longest part).
-//   C = 8: the two K halves of an instruction are two neighbouring taps (the same plane 16 bytes further on).
+//   C = 8: the two K halves of an instruction are two taps, their distance in the plane the descriptor's leading
+//   offset (16 bytes, or to the next row of taps); the ninth tap's partner is a block of zeros with zero weights, so no
+//   pixel outside an output's nine taps enters its sum, were it infinite.
 //   pool: the input is read as the 2x2 average of a tensor of twice the height and width.
 //   skip: the input is [nearest-upsampled in (Cu channels), skip] (a decoder level).
 // Bound by latency: a layer is a few microseconds of loads, instructions and stores between two launches.  The im2col
@@ -45,9 +47,11 @@ struct ConvArgs {
     int R, tiles, plane, cols;
 };
 
-// Shared memory of a CTA: weights, then input planes.
+// Shared memory of a CTA: weights (16-byte chunks, an even number), input planes, and for C = 8 the ninth tap's zeros.
+constexpr int kConvZeros = 128 * 16;
+__host__ __device__ inline int conv_chunks(int C) { return C == 8 ? 10 : 9 * (C / 8); }
 inline size_t conv_smem(int C, int nb, int plane) {
-    return (size_t)(C == 8 ? 12 : 9 * (C / 8)) * nb * 16 + (size_t)(C / 8) * plane * 16;
+    return (size_t)conv_chunks(C) * nb * 16 + (size_t)(C / 8) * plane * 16 + (C == 8 ? kConvZeros : 0);
 }
 
 // Rows a band for B images at nb channels a CTA: the least of a launch's fixed latency per wave, the bytes each SM brings
@@ -59,7 +63,7 @@ constexpr size_t kConvSmem = 226 * 1024;
 constexpr double kConvNone = 1e30;
 inline double conv_plan(ConvArgs &g, int B, int nb) {
     if (g.C % 16 && g.C != 8) return kConvNone;
-    const int wp = g.W + 2, nblk = (g.N + nb - 1) / nb, steps = g.C == 8 ? 6 : 9 * (g.C / 16);
+    const int wp = g.W + 2, nblk = (g.N + nb - 1) / nb, steps = conv_chunks(g.C) / 2;
     double best = kConvNone;
     for (int R = 1; R <= g.H; ++R) {
         const int tiles = (R * wp + 127) / 128;
@@ -97,7 +101,8 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3(const __grid_constant__ 
     const int y0 = blockIdx.x * g.R, rows = min(g.R, g.H - y0);
     const int tiles = (rows * wp + 127) / 128, issuers = min(tiles, kConvThreads / 32);
     const long long img = blockIdx.y;
-    const uint32_t sB = smem_u32(g_umma_smem), sA = sB + (uint32_t)((g.C == 8 ? 12 : 9 * c8) * NB * 16);
+    const uint32_t sB = smem_u32(g_umma_smem), sA = sB + (uint32_t)(conv_chunks(g.C) * NB * 16),
+                   sZ = sA + (uint32_t)(c8 * g.plane * 16);
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&bar)), "r"(issuers));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -105,21 +110,21 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3(const __grid_constant__ 
         abort_flag = 0;
     }
     // weights and bias, before the wait on the previous kernel: they are written by k_cnn_weights and k_cnn_adam, which
-    // lie at least one whole kernel before it in the stream.  Chunk (tap, 8 channels) of output channel n: [chunk][n] of 16 bytes; for
-    // C = 8 the chunks of a row of taps are dx = 0, 1, 2 and one of zeros.  Two chunks of 16 channels a warp.
+    // lie at least one whole kernel before it in the stream.  Chunk (tap, 8 channels) of output channel n: [chunk][n] of
+    // 16 bytes; for C = 8 a tenth chunk of zeros.  Two chunks of 16 channels a warp.
     if (tid < NB) sbias[tid] = g.bias && n0 + tid < g.N ? g.bias[n0 + tid] : 0.f;
     {
-        const int k8 = 9 * c8, chunks = g.C == 8 ? 12 : k8;
+        const int k8 = 9 * c8, chunks = conv_chunks(g.C);
         // a thread keeps its channel and its parity of chunk: 2 NB divides the block
         const int r = tid % (2 * NB), n = r >> 1;
         constexpr int kStep = kConvThreads / NB;
         const bool row = n0 + n < g.N;
         const bf16 *src = g.w + (long long)(row ? n0 + n : 0) * k8 * 8;
-        for (int k = 2 * (tid / (2 * NB)) + (r & 1); k < chunks; k += kStep) {  // chunks is even: C = 8 or C % 16 == 0
-            const int from = g.C == 8 ? (k >> 2) * 3 + (k & 3) : k;
-            const bool ok = row && (g.C != 8 || (k & 3) < 3);
-            cp_async16(sB + (uint32_t)((k * NB + n) * 16), ok ? src + from * 8 : g.w, ok ? 16 : 0);
+        for (int k = 2 * (tid / (2 * NB)) + (r & 1); k < chunks; k += kStep) {
+            const bool ok = row && k < k8;
+            cp_async16(sB + (uint32_t)((k * NB + n) * 16), ok ? src + k * 8 : g.w, ok ? 16 : 0);
         }
+        if (g.C == 8 && tid < kConvZeros / 16) cp_async16(sZ + (uint32_t)(tid * 16), g.w, 0);
     }
     pdl_wait();
     pdl_release();
@@ -132,8 +137,6 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3(const __grid_constant__ 
     }
     // input rows y0 - 1 .. y0 + rows, zero outside the image
     {
-        // C = 8 multiplies the pixel after the last by the chunk of zeros: it must be finite
-        if (g.C == 8 && tid == 0) cp_async16(sA + (uint32_t)((rows + 2) * wp * 16), g.in, 0);
         // One 16-byte chunk of a pixel a step: the chunks of a pixel lie side by side in memory, so neighbouring
         // threads take them.  Where 256 is a multiple of c8 a thread keeps its chunk and walks the pixels by additions
         // alone (with a division or two a chunk this loop was the layer's longest part).
@@ -182,28 +185,41 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3(const __grid_constant__ 
     const uint32_t tmem = tmem_slot;
     if (warp < issuers && lane == 0) {
         const uint32_t idesc = umma_idesc_bf16(NB);
-        const bool c_is_8 = g.C == 8;
-        const int per_tap = c_is_8 ? 2 : g.C / 16, taps = c_is_8 ? 3 : 9;
-        // both descriptors' upper words are the tile's constants; the lower words hold the address in 16-byte units
-        const uint64_t da0 = umma_desc(sA, c_is_8 ? 16u : (uint32_t)g.plane * 16u, 128), db0 = umma_desc(sB, NB * 16, 128);
-        const uint32_t ha = (uint32_t)(da0 >> 32), hb = (uint32_t)(db0 >> 32), stepA = c_is_8 ? 2u : 2u * (uint32_t)g.plane;
+        // both descriptors' upper words are constants; the lower words hold the address and, from bit 16 on, the distance
+        // of the K halves, in 16-byte units
+        const uint64_t da0 = umma_desc(sA, 0, 128), db0 = umma_desc(sB, NB * 16, 128);
+        const uint32_t ha = (uint32_t)(da0 >> 32), hb = (uint32_t)(db0 >> 32);
+        auto mma = [&](uint32_t d, uint32_t a, uint32_t b, uint32_t acc) {
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t.reg .b64 x, y;\n\t"
+                "setp.ne.b32 p, %6, 0;\n\t"
+                "mov.b64 x, {%1, %2};\n\t"
+                "mov.b64 y, {%3, %4};\n\t"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %5, p;\n\t}"
+                :
+                : "r"(d), "r"(a), "r"(ha), "r"(b), "r"(hb), "r"(idesc), "r"(acc));
+        };
         for (int t = warp; t < tiles; t += kConvThreads / 32) {
             const uint32_t d = tmem + (uint32_t)(t * NB);
             uint32_t b = (uint32_t)db0, acc = 0;
-            for (int tap = 0; tap < taps; ++tap) {
-                uint32_t a = (uint32_t)da0 + (uint32_t)(t * 128 + (c_is_8 ? tap * wp : (tap / 3) * wp + tap % 3));
+            if (g.C == 8) {
+#pragma unroll
+                for (int tap = 0; tap < 9; tap += 2) {
+                    const uint32_t at = (uint32_t)(t * 128 + (tap / 3) * wp + tap % 3);
+                    const uint32_t half = tap == 8 ? ((sZ - sA) >> 4) - at
+                                                   : (uint32_t)(((tap + 1) / 3 - tap / 3) * wp + (tap + 1) % 3 - tap % 3);
+                    mma(d, ((uint32_t)da0 + at) | half << 16, b, tap != 0);
+                    b += 2 * NB;
+                }
+                continue;
+            }
+            for (int tap = 0; tap < 9; ++tap) {
+                uint32_t a = ((uint32_t)da0 + (uint32_t)(t * 128 + (tap / 3) * wp + tap % 3)) | (uint32_t)g.plane << 16;
 #pragma unroll 2
-                for (int k = 0; k < per_tap; ++k) {
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\t.reg .b64 x, y;\n\t"
-                        "setp.ne.b32 p, %6, 0;\n\t"
-                        "mov.b64 x, {%1, %2};\n\t"
-                        "mov.b64 y, {%3, %4};\n\t"
-                        "tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %5, p;\n\t}"
-                        :
-                        : "r"(d), "r"(a), "r"(ha), "r"(b), "r"(hb), "r"(idesc), "r"(acc));
+                for (int k = 0; k < g.C / 16; ++k) {
+                    mma(d, a, b, acc);
                     acc = 1;
-                    a += stepA;
+                    a += 2u * (uint32_t)g.plane;
                     b += 2 * NB;
                 }
             }
