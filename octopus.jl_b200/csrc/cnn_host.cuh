@@ -153,9 +153,24 @@ struct Cnn {
         weights_dirty = false;
     }
 
+    // Parts of K in which layer l's sums over a batch of B are added, in order, and the 64-wide chunks of each but the
+    // last: where a GEMM's 128-row output tiles are too few to fill the GPU (the coarse levels), enough to fill it
+    // twice, no shorter than two chunks.
+    struct Parts {
+        int n, chunks;
+    };
+    Parts conv_parts(int l, int B) const {
+        const LayerSpec &L = kLayers[l];
+        const long long tiles = (ml(L.level, B) + kBM - 1) / kBM;  // one column of tiles: cout <= 256
+        const int chunks = (9 * L.cin + kBK - 1) / kBK;
+        const int splits = (l != L_HEAD && tiles < 148 && chunks >= 4)
+                               ? (int)std::min<long long>(chunks / 2, (296 + tiles - 1) / tiles) : 1;
+        const int per = (chunks + splits - 1) / splits;
+        return Parts{(chunks + per - 1) / per, per};
+    }
+
     // A 3x3 convolution layer: by bands of the image (k_conv.cuh), or where no band fits a CTA as one im2col GEMM,
-    // whose layers with too few output tiles to fill the GPU (the coarse levels) split K over more CTAs, their fp32
-    // partials summed in a fixed order by the bias / ReLU / bf16 epilogue kernel.
+    // which takes the parts of K on CTAs of their own, their fp32 sums added by the bias / ReLU / bf16 epilogue kernel.
     // skip != null: the layer's input is [nearest-upsampled in (cu channels), skip] (a decoder level), read
     // directly instead of a materialised concatenation.  pooled != null: the layer's input is the 2x2 average of in;
     // a GEMM takes it from pooled, which this then fills.
@@ -169,6 +184,8 @@ struct Cnn {
         c.bias = master.p + boff[l]; c.relu = L.relu;
         c.out_bf16 = out_bf; c.out = out_f;
         c.error = err;
+        const Parts parts = conv_parts(l, B);
+        c.parts = parts.n; c.part_steps = parts.chunks * (kBK / 16);
         if (launch_conv(c, B, st)) return;
         if (pooled) {
             pool(in, pooled, B, L.level - 1, L.cin, st);
@@ -188,17 +205,13 @@ struct Cnn {
         a.out_bf16 = out_bf; a.ldo = L.cout;
         a.out = out_f; a.ldc = L.cout; a.split_stride = 0; a.k_per_split = ((a.K + kBK - 1) / kBK) * kBK;
         a.error = err;
-        const int bn = L.cout <= 32 ? 32 : (L.cout <= 64 ? 64 : (L.cout <= 128 ? 128 : 256));
-        const long long tiles = ((long long)(a.M + kBM - 1) / kBM) * ((L.cout + bn - 1) / bn);
-        const int chunks = (a.K + kBK - 1) / kBK;
-        const int splits = (out_bf && tiles < 148 && chunks >= 4)
-                               ? (int)std::min<long long>(chunks / 2, (296 + tiles - 1) / tiles) : 1;
-        if (splits <= 1) {
+        const Parts parts = conv_parts(l, B);
+        const int used = parts.n;
+        if (used == 1) {
             launch_gemm(a, 1, st);
             return;
         }
-        a.k_per_split = ((chunks + splits - 1) / splits) * kBK;
-        const int used = (chunks * kBK + a.k_per_split - 1) / a.k_per_split;
+        a.k_per_split = parts.chunks * kBK;
         splitbuf.ensure((size_t)used * a.M * L.cout);
         a.out = splitbuf.p; a.ldc = L.cout; a.split_stride = (long long)a.M * L.cout;
         a.out_bf16 = nullptr; a.bias = nullptr; a.relu = 0;
@@ -301,6 +314,7 @@ struct Cnn {
         c.in = g.p; c.H = hl(L.level); c.W = wl(L.level); c.C = L.cout;
         c.w = wf[l].p; c.N = L.cin;
         c.out = fa.p;
+        c.parts = 1; c.part_steps = 9 * (L.cout / 16);
         c.error = err;
         if (launch_conv(c, B, st)) return;
         GemmArgs a{};

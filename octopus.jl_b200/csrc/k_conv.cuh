@@ -6,18 +6,22 @@
 // no-swizzle K-major layout with 8-row groups 128 bytes apart, so the A operand of a tap is the same planes read from
 // a start address 16 bytes x (dy (W + 2) + dx) further on: no im2col is written or loaded.  Row o = y (W + 2) + x of
 // the product is output pixel (y, x); the two columns x >= W of each row are computed and dropped (4 % at W = 48).
-// The weights of the CTA's NB output channels lie beside it in the same form.  Warp t's first lane issues every
-// tcgen05.mma (M = 128 pixels, N = NB, K = 16) of tile t into TMEM and commits once; an instruction's operands are two
-// additions away from the one before (rebuilt descriptors made the issuing lane the layer's longest part).
+// The weights of the CTA's NB output channels lie beside it in the same form.  A warp's first lane issues every
+// tcgen05.mma (M = 128 pixels, N = NB, K = 16) of its share of the tiles' parts of K into TMEM and commits once; an
+// instruction's operands are two additions away from the one before (rebuilt descriptors made the issuing lane the
+// layer's longest part).
 //   C = 8: the two K halves of an instruction are two taps, their distance in the plane the descriptor's leading
 //   offset (16 bytes, or to the next row of taps); the ninth tap's partner is a block of zeros with zero weights, so no
 //   pixel outside an output's nine taps enters its sum, were it infinite.
+//   parts: where the im2col GEMM of a small layer splits K, a tile has an accumulator for each of its parts, issued by
+//   warps of their own, and the epilogue adds them in order: a layer's fp32 sums are the GEMM's to the bit, whichever of
+//   the two runs it.
 //   pool: the input is read as the 2x2 average of a tensor of twice the height and width.
 //   skip: the input is [nearest-upsampled in (Cu channels), skip] (a decoder level).
 // Bound by latency: a layer is a few microseconds of loads, instructions and stores between two launches.  The im2col
 // GEMM (k_umma.cuh) reads every input nine times in K chunks that wait for one another: a forward pass over 20 planes of
-// 48 x 48 took 304 us with it (split-K folds and pools included) and takes 160 us; a
-// batch-64 training step took 2.01 ms with it, 1.57 ms with the first form of this kernel.
+// 48 x 48 took 304 us with it (split-K folds and pools included) and takes 167 us (158 with each layer's sum in one part:
+// the accumulators of the parts take TMEM, and the second 128-channel layer runs a second wave of CTAs).
 //
 // The mbarrier wait is bounded (about one second of the global timer); on expiry the kernel records OCTO_ERR_TIMEOUT
 // in *error, frees its TMEM and returns.
@@ -42,6 +46,7 @@ struct ConvArgs {
     int relu;
     bf16 *out_bf16;          // bf16 result, or null:
     float *out;              // fp32 result
+    int parts, part_steps;   // parts of K (C = 8: one) and the 16-channel steps of each but the last
     int *error;
     // the split (conv_plan): rows a band, 128-row tiles a band, pixels of a plane (odd), TMEM columns
     int R, tiles, plane, cols;
@@ -55,7 +60,7 @@ inline size_t conv_smem(int C, int nb, int plane) {
 }
 
 // Rows a band for B images at nb channels a CTA: the least of a launch's fixed latency per wave, the bytes each SM brings
-// in and the instructions it issues, over the bands that fit (half of TMEM, so that two CTAs share an SM, and kConvSmem:
+// in and the instructions it issues, over the bands that fit (TMEM, half of it for a sum in one part, and kConvSmem:
 // 227 KB less the 1 KB of this kernel itself).  Returns that cost (about a microsecond a unit), 1e30 when none fits (very
 // wide images: the im2col GEMM runs those).  While bands were held to 200 KB the widest decoder layer (256 to 64
 // channels, 12 x 12, 20 images) ran 240 CTAs in two waves, 31 us; now one band an image, 80 CTAs, 19 us.
@@ -67,12 +72,12 @@ inline double conv_plan(ConvArgs &g, int B, int nb) {
     double best = kConvNone;
     for (int R = 1; R <= g.H; ++R) {
         const int tiles = (R * wp + 127) / 128;
-        if (tiles * nb > 256) break;
+        if (tiles * nb * g.parts > (g.parts == 1 ? 256 : 512)) break;
         const int plane = (tiles * 128 + 2 * wp + 4) | 1;
         const size_t smem = conv_smem(g.C, nb, plane);
         if (smem > kConvSmem) break;
         int cols = 32;
-        while (cols < tiles * nb) cols *= 2;
+        while (cols < tiles * nb * g.parts) cols *= 2;
         const long long ctas = (long long)((g.H + R - 1) / R) * B * nblk;
         const int res = (int)std::min<long long>({(long long)(228 * 1024 / (smem + 2048)), 512 / cols, 8});
         const double per_sm = (double)((ctas + 147) / 148), waves = (double)((ctas + 148LL * res - 1) / (148LL * res));
@@ -99,7 +104,7 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3(const __grid_constant__ 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int c8 = g.C / 8, n0 = blockIdx.z * NB, wp = g.W + 2;
     const int y0 = blockIdx.x * g.R, rows = min(g.R, g.H - y0);
-    const int tiles = (rows * wp + 127) / 128, issuers = min(tiles, kConvThreads / 32);
+    const int tiles = (rows * wp + 127) / 128, units = tiles * g.parts, issuers = min(units, kConvThreads / 32);
     const long long img = blockIdx.y;
     const uint32_t sB = smem_u32(g_umma_smem), sA = sB + (uint32_t)(conv_chunks(g.C) * NB * 16),
                    sZ = sA + (uint32_t)(c8 * g.plane * 16);
@@ -199,9 +204,11 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3(const __grid_constant__ 
                 :
                 : "r"(d), "r"(a), "r"(ha), "r"(b), "r"(hb), "r"(idesc), "r"(acc));
         };
-        for (int t = warp; t < tiles; t += kConvThreads / 32) {
-            const uint32_t d = tmem + (uint32_t)(t * NB);
-            uint32_t b = (uint32_t)db0, acc = 0;
+        const int per_tap = g.C / 16, steps = 9 * per_tap;
+        for (int u = warp; u < units; u += kConvThreads / 32) {
+            const int t = u / g.parts, s0 = (u - t * g.parts) * g.part_steps, s1 = min(steps, s0 + g.part_steps);
+            const uint32_t d = tmem + (uint32_t)(u * NB);
+            uint32_t b = (uint32_t)db0 + (uint32_t)(s0 * 2 * NB), acc = 0;
             if (g.C == 8) {
 #pragma unroll
                 for (int tap = 0; tap < 9; tap += 2) {
@@ -213,10 +220,14 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3(const __grid_constant__ 
                 }
                 continue;
             }
-            for (int tap = 0; tap < 9; ++tap) {
-                uint32_t a = ((uint32_t)da0 + (uint32_t)(t * 128 + (tap / 3) * wp + tap % 3)) | (uint32_t)g.plane << 16;
+            int tap = s0 / per_tap, k = s0 - tap * per_tap;
+            for (int s = s0; s < s1; ++tap, k = 0) {
+                uint32_t a = ((uint32_t)da0 + (uint32_t)(t * 128 + (tap / 3) * wp + tap % 3 + 2 * k * g.plane)) |
+                             (uint32_t)g.plane << 16;
+                const int run = min(per_tap - k, s1 - s);
+                s += run;
 #pragma unroll 2
-                for (int k = 0; k < g.C / 16; ++k) {
+                for (int i = 0; i < run; ++i) {
                     mma(d, a, b, acc);
                     acc = 1;
                     a += 2u * (uint32_t)g.plane;
@@ -233,37 +244,44 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3(const __grid_constant__ 
     if (abort_flag) {
         if (tid == 0 && g.error) atomicExch(g.error, kTimeoutCode);
     } else {
-        // warp w reads TMEM lanes 32 (w % 4) .. + 31 of every other tile; a lane holds one pixel's NB channels
+        // warp w reads TMEM lanes 32 (w % 4) .. + 31 of every other tile; a lane holds one pixel, 16 channels at a time
         for (int t = warp >> 2; t < tiles; t += 2) {
-            __syncwarp();
-            uint32_t r[NB];
-            const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(t * NB);
-#pragma unroll
-            for (int h = 0; h < NB; h += 16)
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-                    "%14, %15}, [%16];"
-                    : "=r"(r[h + 0]), "=r"(r[h + 1]), "=r"(r[h + 2]), "=r"(r[h + 3]), "=r"(r[h + 4]), "=r"(r[h + 5]),
-                      "=r"(r[h + 6]), "=r"(r[h + 7]), "=r"(r[h + 8]), "=r"(r[h + 9]), "=r"(r[h + 10]), "=r"(r[h + 11]),
-                      "=r"(r[h + 12]), "=r"(r[h + 13]), "=r"(r[h + 14]), "=r"(r[h + 15])
-                    : "r"(taddr + (uint32_t)h));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int e = 0; e < NB; ++e) asm volatile("" : "+r"(r[e]));  // the values exist from here on
             const int o = t * 128 + (warp & 3) * 32 + lane, y = o / wp, x = o - y * wp;
-            if (y >= rows || x >= g.W) continue;
+            const bool in = y < rows && x < g.W;
             const long long m = (img * g.H + y0 + y) * g.W + x;
+            const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(t * g.parts * NB);
 #pragma unroll
-            for (int h = 0; h < NB; h += 8) {
-                if (n0 + h >= g.N) break;  // N is a multiple of 8
-                float v[8];
+            for (int c = 0; c < NB; c += 16) {
+                __syncwarp();
+                float sum[16];
+                for (int z = 0; z < g.parts; ++z) {
+                    uint32_t r[16];
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                        "%14, %15}, [%16];"
+                        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
+                          "=r"(r[15])
+                        : "r"(taddr + (uint32_t)(z * NB + c)));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    v[e] = __uint_as_float(r[h + e]) + sbias[h + e];
-                    if (g.relu) v[e] = fmaxf(v[e], 0.f);
+                    for (int e = 0; e < 16; ++e) {
+                        asm volatile("" : "+r"(r[e]));  // the values exist from here on
+                        sum[e] = z ? sum[e] + __uint_as_float(r[e]) : __uint_as_float(r[e]);
+                    }
                 }
-                if (g.out_bf16) store_bf8(g.out_bf16 + m * g.N + n0 + h, v);
-                else store_f8(g.out + m * g.N + n0 + h, v);
+#pragma unroll
+                for (int h = 0; h < 16; h += 8) {
+                    if (!in || n0 + c + h >= g.N) break;  // N is a multiple of 8
+                    float v[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        v[e] = sum[h + e] + sbias[c + h + e];
+                        if (g.relu) v[e] = fmaxf(v[e], 0.f);
+                    }
+                    if (g.out_bf16) store_bf8(g.out_bf16 + m * g.N + n0 + c + h, v);
+                    else store_f8(g.out + m * g.N + n0 + c + h, v);
+                }
             }
         }
     }

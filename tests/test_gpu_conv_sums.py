@@ -1,6 +1,6 @@
 """The band convolutions of the network's forward pass against the same layers as im2col GEMMs of the same tensor cores
-(octo_gemm_bf16): K is taken 16 at a time, tap by tap and channel by channel, so where the GEMM does not split K
-every layer's fp32 sums, and with them the bf16 activations and the output, agree to the bit.
+(octo_gemm_bf16): K is taken 16 at a time, tap by tap and channel by channel, and where the GEMM would split K its parts
+are summed in order, so every layer's fp32 sums, and with them the bf16 activations and the output, agree to the bit.
 Infinities and NaN too: an input pixel reaches the outputs whose nine taps hold it and no other."""
 import ctypes as C
 
@@ -90,4 +90,11 @@ def _check(B, H, W, odd):
 @pytest.mark.parametrize("odd", [False, True])
 @pytest.mark.parametrize("B,H,W", [(74, 128, 128), (400, 64, 48)])
 def test_layers_whose_tiles_fill_the_device(B, H, W, odd):
+    _check(B, H, W, odd)
+
+
+@pytest.mark.parametrize("odd", [False, True])
+@pytest.mark.parametrize("B,H,W", [(20, 48, 48), (1, 48, 48), (64, 32, 32), (1, 16, 16), (5, 40, 24), (3, 16, 64),
+                                   (70, 48, 48)])
+def test_layers_in_parts(B, H, W, odd):
     _check(B, H, W, odd)
