@@ -93,6 +93,7 @@ inline double conv_plan(ConvArgs &g, int B, int nb) {
     return best;
 }
 
+// grid (bands of an image x images, ceil(N / NB)): the images lie on x, whose limit no batch reaches.
 template <int NB>
 __global__ void __launch_bounds__(kConvThreads) k_conv3(const __grid_constant__ ConvArgs g) {
     static_assert(NB == 16 || NB == 32, "NB");
@@ -102,10 +103,10 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3(const __grid_constant__ 
     __shared__ int abort_flag;
     __shared__ float sbias[NB];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int c8 = g.C / 8, n0 = blockIdx.z * NB, wp = g.W + 2;
-    const int y0 = blockIdx.x * g.R, rows = min(g.R, g.H - y0);
+    const int c8 = g.C / 8, n0 = blockIdx.y * NB, wp = g.W + 2;
+    const int bands = (g.H + g.R - 1) / g.R, y0 = (int)(blockIdx.x % bands) * g.R, rows = min(g.R, g.H - y0);
     const int tiles = (rows * wp + 127) / 128, units = tiles * g.parts, issuers = min(units, kConvThreads / 32);
-    const long long img = blockIdx.y;
+    const long long img = blockIdx.x / bands;
     const uint32_t sB = smem_u32(g_umma_smem), sA = sB + (uint32_t)(conv_chunks(g.C) * NB * 16),
                    sZ = sA + (uint32_t)(c8 * g.plane * 16);
     if (tid == 0) {

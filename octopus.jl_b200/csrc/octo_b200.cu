@@ -264,7 +264,7 @@ bool launch_conv(ConvArgs g, int B, cudaStream_t st) {
     const int nb = wide_cost <= narrow_cost ? 32 : 16;
     if (nb == 32) g = wide;
     const size_t smem = conv_smem(g.C, nb, g.plane);
-    const dim3 grid((unsigned)((g.H + g.R - 1) / g.R), (unsigned)B, (unsigned)((g.N + nb - 1) / nb));
+    const dim3 grid((unsigned)((long long)((g.H + g.R - 1) / g.R) * B), (unsigned)((g.N + nb - 1) / nb));
     void (*kernel)(const ConvArgs) = nb == 16 ? k_conv3<16> : k_conv3<32>;
     CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kConvSmem));
     CK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));

@@ -98,3 +98,7 @@ def test_layers_whose_tiles_fill_the_device(B, H, W, odd):
                                    (70, 48, 48)])
 def test_layers_in_parts(B, H, W, odd):
     _check(B, H, W, odd)
+
+
+def test_more_images_than_a_grid_axis_takes():
+    _check(65537, 16, 16, False)
