@@ -24,7 +24,7 @@
 // the accumulators of the parts take TMEM, and the second 128-channel layer runs a second wave of CTAs).
 //
 // The mbarrier wait is bounded (about one second of the global timer); on expiry the kernel records OCTO_ERR_TIMEOUT
-// in *error, frees its TMEM and returns.
+// in *error after a second such wait for the instructions in flight, frees its TMEM and returns.
 #pragma once
 #include <algorithm>
 
@@ -239,7 +239,10 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3(const __grid_constant__ 
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&bar))
                      : "memory");
     }
-    if (tid == 0 && !mbar_wait(smem_u32(&bar), 0)) abort_flag = 1;
+    if (tid == 0 && !mbar_wait(smem_u32(&bar), 0)) {
+        mbar_wait(smem_u32(&bar), 0);
+        abort_flag = 1;
+    }
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (abort_flag) {
