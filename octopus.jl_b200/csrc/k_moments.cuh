@@ -7,9 +7,10 @@
 // products, and k_moment_finish turns them into the means and the second central moments, m_ij = S_ij / n - d_i d_j
 // with d = S / n the mean's offset from the pivot.  The definition takes the means first, in a pass of its own; one
 // read of the beam instead of two, and three launches instead of six, took the rows of a 2.56M and a 1.024M-particle
-// float64 beam from 128 to 65 us of kernel time together (26 us of reading at the measured copy bandwidth).  The pivot (k_moment_pivot) is zero for
-// a centred coordinate, where d is the mean itself, and else the mean of 4096 particles spread over the beam, about
-// sigma / 64 from the mean and at most sqrt(n) / 4096 of the sigma that a stray particle makes; either way the
+// float64 beam from 128 to 65 us of kernel time together (26 us of reading at the measured copy bandwidth).  The pivot
+// (k_moment_pivot) is zero for a centred coordinate, where d is the mean itself, and else the mean of 4096 particles
+// spread over the beam (its live ones when lost particles are masked), about sigma / 64 from the mean and at most
+// sqrt(n) / 4096 of the sigma that a stray particle makes; either way the
 // subtraction loses nothing.  (Zero matters: a mean far smaller than sigma would be the sum of a pivot and its
 // opposite, which costs it three digits.)  Rows of order 3 and more (k_moment_general) read the beam
 // again, in chunks, with the means known.  Each pass writes per-block partials (a fixed block count) that are summed
@@ -90,48 +91,75 @@ struct MomentBeam {
     int mask;
 };
 
-// Block d: coordinate d's pivot from its finite values among 4096 particles spread over the beam: their mean, or zero
-// when there is none or the mean lies within an eighth of their rms spread.
+// Block d: coordinate d's pivot from 4096 particles spread over the beam, of them the live ones when lost particles are
+// masked and else those with a finite value: their mean, or zero when there is none or the mean lies within an eighth of
+// their rms spread.  (A lost particle's other coordinates can be anything: taken in, they would put the pivot far from
+// the live beam, where the row's differences cancel.)  When every sample is lost, the next live particles of the
+// whole beam take their place, which a beam with few of them or none pays for with up to one read of it.
 constexpr int kPivotThreads = 1024, kPivotPer = 4;
 template <class R>
 __global__ void __launch_bounds__(kPivotThreads) k_moment_pivot(const __grid_constant__ MomentBeam<R> B, double *pivot) {
     pdl_wait();
     pdl_release();
     __shared__ double red[3][kPivotThreads / 32];
+    __shared__ double total[3];
     const R *c = B.c[blockIdx.x];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double v[kPivotPer], s[3] = {0.0, 0.0, 0.0};  // sum, sum of squares, count
+    constexpr long long kSamples = kPivotThreads * kPivotPer;
+    // the sum, the sum of squares and the count of kSamples particles' values, particle(q) the q-th one's index
+    auto gather = [&](auto particle) {
+        double v[kPivotPer], s[3] = {0.0, 0.0, 0.0};
+        bool on[kPivotPer];
 #pragma unroll
-    for (int k = 0; k < kPivotPer; ++k) {
-        const long long q = (long long)k * kPivotThreads + threadIdx.x, samples = kPivotThreads * kPivotPer;
-        // every particle of a small beam once, else 4096 of them (q n / 4096 without the product's overflow)
-        const long long i = B.n <= samples ? q : B.n / samples * q + B.n % samples * q / samples;
-        v[k] = i < B.n ? (double)c[i] : (double)NAN;
-    }
-#pragma unroll
-    for (int k = 0; k < kPivotPer; ++k)
-        if (isfinite(v[k])) {
-            s[0] += v[k];
-            s[1] = fma(v[k], v[k], s[1]);
-            s[2] += 1.0;
+        for (int k = 0; k < kPivotPer; ++k) {
+            const long long i = particle((long long)k * kPivotThreads + threadIdx.x);
+            on[k] = i < B.n;
+            v[k] = on[k] ? (double)c[i] : 0.0;
+            if (B.mask && on[k]) {
+                double p[6];
+                load6(p, B.c[0], B.c[1], B.c[2], B.c[3], B.c[4], B.c[5], i);
+                on[k] = live6(p);
+            }
         }
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
+        for (int k = 0; k < kPivotPer; ++k)
+            if (on[k] && isfinite(v[k])) {
+                s[0] += v[k];
+                s[1] = fma(v[k], v[k], s[1]);
+                s[2] += 1.0;
+            }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
-        if (lane == 0) red[k][warp] = s[k];
-    }
-    __syncthreads();
-    if (warp) return;
+        for (int k = 0; k < 3; ++k) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        s[k] = red[k][lane];
+            for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+            if (lane == 0) red[k][warp] = s[k];
+        }
+        __syncthreads();
+        if (warp == 0) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
-    }
-    const double mean = s[0] / s[2];
-    const bool centred = 65.0 * mean * mean <= s[1] / s[2];  // mean^2 <= (mean square - mean^2) / 64
-    if (lane == 0) pivot[blockIdx.x] = isfinite(mean) && !centred ? mean : 0.0;
+            for (int k = 0; k < 3; ++k) {
+                s[k] = red[k][lane];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+                if (lane == 0) total[k] = s[k];
+            }
+        }
+        __syncthreads();
+    };
+    // every particle of a small beam once, else 4096 of them (q n / 4096 without the product's overflow); with lost ones
+    // masked, 128 runs of 32 neighbours, whose six loads a particle coalesce (one by one they took 12 us)
+    constexpr long long kRuns = kSamples / 32;
+    gather([&](long long q) {
+        if (B.n <= kSamples) return q;
+        const long long m = B.mask ? kRuns : kSamples, g = B.mask ? q / 32 : q;
+        return B.n / m * g + B.n % m * g / m + (B.mask ? q % 32 : 0);
+    });
+    if (B.mask && B.n > kSamples)
+        for (long long k = 0; k < B.n && total[2] == 0.0; k += kSamples) gather([&](long long q) { return k + q; });
+    if (threadIdx.x != 0) return;
+    const double mean = total[0] / total[2], square = total[1] / total[2];
+    const bool centred = isfinite(square) && 65.0 * mean * mean <= square;  // mean^2 <= (square - mean^2) / 64
+    pivot[blockIdx.x] = isfinite(mean) && !centred ? mean : 0.0;
 }
 
 // Bound by HBM with 56 of its registers holding sums: two blocks per SM, and the next two particles' twelve loads

@@ -71,3 +71,40 @@ def test_non_finite_samples_leave_the_pivot(bad):
         else:
             assert np.isfinite(rows[False][k])
     torch.cuda.synchronize()
+
+
+def _live_row(c, dtype):
+    """Row of a masked observer and the extended-precision moments of its live particles."""
+    import octo_b200 as ob
+    c = c.astype(np.float32).astype(np.float64) if dtype == torch.float32 else c
+    obs = ob.MomentObserver("b", orders=(1, 2), mask_lost=True)
+    obs.observe(0, ob.Beam.from_numpy(c, ob.BeamParams(1.0, 1.0, 1.0, 1.0, 1.0), dtype=dtype))
+    return obs.rows()[0], c[:, np.isfinite(c).all(axis=0)].astype(np.longdouble)
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("far", [1e4, 1e10])
+@pytest.mark.parametrize("case", ["one in twenty", "every sample", "three left", "one left"])
+def test_lost_particles_leave_the_pivot(case, far, dtype):
+    """A lost particle (one coordinate NaN or infinite) may hold any finite values in the others: they are no part of a
+    masked row, so they must not move the pivot away from the live particles either."""
+    n = 200_000
+    c = _beam("plain" if case == "one in twenty" else "offset", n)
+    lost = {"one in twenty": np.arange(0, n, 20), "every sample": np.arange(n)[np.arange(n) % 17 != 5],
+            "three left": np.setdiff1d(np.arange(n), [77_777, 77_779, 150_000]),
+            "one left": np.setdiff1d(np.arange(n), [199_999])}[case]
+    c[:, lost] = far
+    c[3, lost] = np.nan
+    c[3, lost[::2]] = np.inf
+    row, live = _live_row(c, dtype)
+    mean = live.mean(axis=1)
+    d = live - mean[:, None]
+    rms = np.sqrt((d * d).mean(axis=1))
+    # the bounds of test_row_matches_extended_precision
+    np.testing.assert_array_less(np.abs(row[1:7] - mean), 1e-13 * rms + 2.3e-16 * np.abs(mean) + 1e-300)
+    k = 7
+    for i in range(6):
+        for j in range(i, 6):
+            own = 1e-32 * abs(mean[i] * mean[j])
+            assert abs(row[k] - (d[i] * d[j]).mean()) <= 1e-13 * rms[i] * rms[j] + own + 1e-300, (i, j, row[k])
+            k += 1
