@@ -17,6 +17,7 @@
 // operations, so they are identical to the reference's values.
 #pragma once
 #include "octo_internal.cuh"
+#include "residual.h"
 #include "k_misc.cuh"
 
 namespace octo {
@@ -47,7 +48,7 @@ constexpr int kPlanar = 1;
 
 // One compiled element.  a[] layout per kind:
 //   Linear6D   a[0..35] row-major matrix
-//   crab       a[h] i kcc, a[8+h] strengthX, a[16+h] strengthY, a[24+h] phase (h < n); rec[h] 1 / (i kcc), h < 6
+//   crab       a[h] i kcc, a[8+h] strengthX, a[16+h] strengthY, a[24+h] phase (h < n); rec[h] 1 / (i kcc), h < nrec
 //   boost      a[0] cos, a[1] sin, a[2] tan of the half crossing angle; rec[0] 1 / cos, rec[1] 1 / cos^2
 //   chrom      a[0..1] xi, a[2..3] beta, a[4..5] alpha, a[6..7] gamma, a[8..11] zeta, a[12..15] eta,
 //              a[16..19] R, a[20] 1/sqrt(1 + r1 r4 - r2 r3)
@@ -55,7 +56,7 @@ constexpr int kPlanar = 1;
 //              flags: kRadDamping | kRadExcitation (effective components); key[c]: component c+1's key
 //   crab disp  a[0..3] zeta;  mom disp a[0..3] eta;  xy a[0..3] r, a[4] g, n = mode
 struct LineOp {
-    int kind, n, flags, pad;
+    int kind, n, flags, nrec;
     double a[36];
     union {
         unsigned long long key[6];
@@ -133,13 +134,6 @@ __device__ __forceinline__ void xy_coupling_inv_a(Coords &c, const double *r, do
 
 __device__ __forceinline__ bool all_finite6(const Coords &c) { return isfinite(c.x + c.px + c.y + c.py + c.z + c.pz); }
 
-// x / d as the division rounds it, rd = 1 / d rounded: a product, its residual and one correction, where the division
-// makes its own reciprocal each time.  A quotient that overflows or is not a number stays what the product is.
-__device__ __forceinline__ double quotient(double x, double d, double rd) {
-    const double q = x * rd, r = fma(-q, d, x);
-    return r == r ? fma(r, rd, q) : q;
-}
-
 __device__ __forceinline__ void linear6d(Coords &c, const double *m, int flags) {
     const double a = c.x, b = c.px, d = c.y, e = c.py, f = c.z, h = c.pz;
     if ((flags & kPlanar) && all_finite6(c)) {
@@ -170,7 +164,7 @@ __device__ __forceinline__ void crab_cavity(Coords &c, const LineOp &op) {
         double s, co;
         sincos(ikcc * c.z + op.a[24 + h], &s, &co);
         const double sx = op.a[8 + h], sy = op.a[16 + h];
-        if (h < 6) {
+        if (h < op.nrec) {
             dpx -= quotient(sx * s, ikcc, op.rec[h]);
             dpy -= quotient(sy * s, ikcc, op.rec[h]);
         } else {

@@ -2267,8 +2267,12 @@ int compile_line_op(const octo_element &e, int rng, uint64_t seed, LineOp &op, s
                 op.a[8 + op.n] = p[1 + h];
                 op.a[16 + op.n] = p[9 + h];
                 op.a[24 + op.n] = p[17 + h];
-                if (op.n < 6) op.rec[op.n] = 1.0 / op.a[op.n];
                 ++op.n;
+            }
+            // reciprocals of the first harmonics up to one whose i kcc is no normal number (a frequency near 1e-300)
+            while (op.nrec < std::min(op.n, 6) && std::isnormal(op.a[op.nrec])) {
+                op.rec[op.nrec] = 1.0 / op.a[op.nrec];
+                ++op.nrec;
             }
             return OCTO_OK;
         }

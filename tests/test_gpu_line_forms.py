@@ -48,3 +48,32 @@ def test_boost_pair(angle):
     from octo_b200 import line as ln
     _check([ln.LorentzBoostSpec(angle)], turns=1)
     _check([ln.RevLorentzBoostSpec(angle)], turns=1)
+
+
+def _same(elems, c):
+    """Finite and infinite values where the oracle has them, of the oracle's values."""
+    got, want = gpu_track(elems, c.copy(), turns=1), oracle_track(elems, c.copy(), turns=1)
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    there = ~np.isnan(want)
+    assert np.array_equal(np.isinf(got), np.isinf(want)) and np.array_equal(np.sign(got[there]), np.sign(want[there]))
+    there &= ~np.isinf(want)
+    np.testing.assert_allclose(got[there], want[there], rtol=1e-14, atol=0)  # a few roundings of each side
+
+
+@pytest.mark.parametrize("angle", [1.2, -0.4])
+def test_boost_quotients_that_overflow(angle):
+    from octo_b200 import line as ln
+    c = np.zeros((6, 8))
+    c[3] = [1.7e308, -1.7e308, 1e-310, 0.0, 5e-324, -1e-300, 1e-3, 1e3]
+    c[4] = [0.0, 1e-3, 1.7e308, -1.7e308, 1e-320, 1e300, 0.0, -0.0]
+    _same([ln.LorentzBoostSpec(angle)], c)
+
+
+@pytest.mark.parametrize("f,strength", [(1.0, 1.6e308), (1e-303, 1e-310), (1e-303, 1e-3), (1e300, 1e-3)])
+def test_crab_quotients_that_overflow(f, strength):
+    from octo_b200 import line as ln
+    c = np.zeros((6, 3))
+    c[0], c[4] = [1e-4, 0.0, -1e-4], [1e-2, 0.0, -3e-2]
+    if f == 1e300:
+        c[4] = 0.0  # the phase alone: no reduction of a huge angle
+    _same([ln.ThinCrabCavitySpec(f, N=2, strengthX=(strength, strength), strengthY=(0.0, -strength), phase=(1.0, -0.5))], c)
