@@ -11,6 +11,7 @@
 // (src/math/SpecialMath.jl:77-157).
 #pragma once
 #include "octo_internal.cuh"
+#include "residual.h"
 
 namespace octo {
 
@@ -83,12 +84,6 @@ __device__ __noinline__ void faddeeva_upper(double zr, double zi, double &wr, do
 
 __device__ __forceinline__ bool faddeeva_is_far(double x, double y) {  // x, y >= 0: faddeeva_upper's own switch
     return y > 7.0 || (x > 6.0 && (y > 0.1 || (x > 8.0 && y > 1e-10) || x > 28.0));
-}
-
-// x / d rounded as the division rounds it, from rd = 1 / d to the last bit: a multiplication and one residual step.
-__device__ __forceinline__ double div_by(double x, double d, double rd) {
-    const double q = x * rd;
-    return fma(fma(-q, d, x), rd, q);
 }
 
 // w at two first-quadrant points of the rational approximation's region: faddeeva_upper's expressions with the two
@@ -396,8 +391,7 @@ struct BeShape {
 // sqrt(v) and a reciprocal of it, v > 0
 __device__ __forceinline__ double sqrt_by(double v, double &rs) {
     rs = rsqrt(v);
-    const double s = v * rs;
-    return fma(fma(-s, s, v), 0.5 * rs, s);
+    return root(v, rs);
 }
 __device__ __forceinline__ BeShape be_shape(double vx, double vy) {  // the variances along x and y, positive
     BeShape S;
@@ -409,8 +403,8 @@ __device__ __forceinline__ BeShape be_shape(double vx, double vy) {  // the vari
     S.d = S.s2 * S.s2;
     r1 = fma(fma(-S.s1, r1, 1.0), r1, r1);
     r2 = fma(fma(-S.s2, r2, 1.0), r2, r2);
-    S.r = div_by(S.s2, S.s1, r1);
-    S.ir = div_by(S.s1, S.s2, r2);
+    S.r = quotient_in_range(S.s2, S.s1, r1);
+    S.ir = quotient_in_range(S.s1, S.s2, r2);
     S.ia = r1 * r1;
     S.id = r2 * r2;
     const double t2 = S.a - S.d;
@@ -418,7 +412,7 @@ __device__ __forceinline__ BeShape be_shape(double vx, double vy) {  // the vari
     S.den = 1.4142135623730951 * sqrt_by(t2, rt);
     rt *= 0.70710678118654752;
     S.iden = fma(fma(-S.den, rt, 1.0), rt, rt);
-    S.A = div_by(2.0 * 1.7724538509055159, S.den, S.iden);
+    S.A = quotient_in_range(2.0 * 1.7724538509055159, S.den, S.iden);
     return S;
 }
 // Kick and potential Hessians per unit kbb along x and y, and e = exp(-(x^2/varx + y^2/vary)/2).
@@ -440,10 +434,11 @@ __device__ __noinline__ BeKick be_general(double sigx, double sigy, double x, do
 }
 // The elliptic response.  A point takes one exponential, the two divisions of faddeeva_pair and about 420 other FP64
 // operations; the general response divides about 28 times and takes two exponentials and five square roots for the
-// same numbers.
+// same numbers.  The point's coordinates are finite and below 1e154 (the moments' check refuses a beam with others); their
+// squares over the variances can overflow, to no density and the kick of a distant charge.
 __device__ __forceinline__ BeKick be_shape_response(const BeShape &S, double px, double py) {
     const double x = S.swap ? py : px, y = S.swap ? px : py;
-    const double rho2 = div_by(x * x, S.a, S.ia) + div_by(y * y, S.d, S.id);
+    const double rho2 = quotient(x * x, S.a, S.ia) + quotient(y * y, S.d, S.id);
     BeKick k;
     // near the axis (be_near_axis, squared and without its division and square roots): the radial series
     const double rho4 = rho2 * rho2;
@@ -452,8 +447,8 @@ __device__ __forceinline__ BeKick be_shape_response(const BeShape &S, double px,
         k.e = exp(-0.5 * rho2);
     } else {
         const double ax = fabs(x), ay = fabs(y);
-        const double z1r = div_by(ax, S.den, S.iden), z1i = div_by(ay, S.den, S.iden);
-        const double z2r = div_by(S.r * ax, S.den, S.iden), z2i = div_by(S.ir * ay, S.den, S.iden);
+        const double z1r = quotient_in_range(ax, S.den, S.iden), z1i = quotient_in_range(ay, S.den, S.iden);
+        const double z2r = quotient_in_range(S.r * ax, S.den, S.iden), z2i = quotient_in_range(S.ir * ay, S.den, S.iden);
         WPair w;
         if (faddeeva_is_far(z1r, z1i) || faddeeva_is_far(z2r, z2i)) w = faddeeva_pair_far(z1r, z1i, z2r, z2i);
         else w = faddeeva_pair(z1r, z1i, z2r, z2i);

@@ -29,12 +29,9 @@ def _probes(sx, sy, n):
     return c
 
 
-@pytest.mark.parametrize("aspect", [1.0, 1.0 + 1e-4, 1.0 + 3e-4, 1.0 + 5e-4, 1.02, 11.0, 1.0 / 11.0, 150.0])
-@pytest.mark.parametrize("n", [441, 3 * 444 * 256 + 77])  # one particle a thread; several, with a ragged last block
-def test_kick_of_every_regime(aspect, n):
+def _collide(e, p):
+    """Luminosity and the probes' coordinates of one pair of single slices, here and (in place) in the oracle."""
     import octo_b200 as ob
-    sy = 1e-5
-    e, p = _source(4001, aspect * sy, sy), _probes(aspect * sy, sy, n)
     solver = ob.GaussianPoissonSolver(slicing=ob.LongitudinalSlicing(nslices=1, method="normal_quantile"), kbb1=1.0,
                                       kbb2=1.0, luminosity_scale=1.0, gaussian_when_luminosity=1)
     params = [ob.BeamParams(q["charge"], q["mass"], q["energy"], q["r0"], q["npart"]) for q in (E_PARAMS, P_PARAMS)]
@@ -42,7 +39,15 @@ def test_kick_of_every_regime(aspect, n):
     lum = ob.collide(solver, be, bp)
     opt = orc.OracleOptions(nslices1=1, nslices2=1, kbb1=1.0, kbb2=1.0, luminosity_scale=1.0)
     ref = orc.gaussian_collide(opt, e, p, *oracle_params(), 0.0, 1, False, False, "hirata", False)
-    got = bp.numpy()
+    return lum, ref, bp.numpy()
+
+
+@pytest.mark.parametrize("aspect", [1.0, 1.0 + 1e-4, 1.0 + 3e-4, 1.0 + 5e-4, 1.02, 11.0, 1.0 / 11.0, 150.0])
+@pytest.mark.parametrize("n", [441, 3 * 444 * 256 + 77])  # one particle a thread; several, with a ragged last block
+def test_kick_of_every_regime(aspect, n):
+    sy = 1e-5
+    e, p = _source(4001, aspect * sy, sy), _probes(aspect * sy, sy, n)
+    lum, ref, got = _collide(e, p)
     assert abs(lum / ref - 1.0) < 1e-12
     # each side rounds w(z) to about 4 x 1.1e-16, and the elliptic form multiplies the difference of two such values by
     # 2 sqrt(pi) / (sqrt(2) sqrt(2 eta) sigma) <= 84 / sigma (eta >= 4.4e-4), where the largest kick is 0.45 / sigma:
@@ -51,3 +56,16 @@ def test_kick_of_every_regime(aspect, n):
         assert np.max(np.abs(got[k] - p[k])) <= 3e-13 * np.max(np.abs(p[[1, 3]]))
     # the longitudinal kick here is the drift term of the kicked momenta alone
     assert np.max(np.abs(got[5] - p[5])) <= 2e-12 * np.max(np.abs(p[5])) + 1e-16
+
+
+@pytest.mark.parametrize("aspect", [11.0, 1.0 / 11.0, 150.0])
+def test_particles_far_outside(aspect):
+    """Coordinates whose square over the variance overflows: no density, and the kick of a distant charge."""
+    sy = 1e-5
+    e, p = _source(4001, aspect * sy, sy), _probes(aspect * sy, sy, 441)
+    p[0, 7], p[2, 9], p[0, 11], p[2, 11] = 1e153, -1e153, -3e152, 2e151
+    lum, ref, got = _collide(e, p)
+    assert np.isfinite(ref) and abs(lum / ref - 1.0) < 1e-12
+    far = [7, 9, 11]
+    assert np.isfinite(got).all() and np.isfinite(p).all()
+    np.testing.assert_allclose(got[:, far], p[:, far], rtol=1e-13, atol=1e-300)

@@ -1,8 +1,9 @@
-"""The quotient by residual correction (octopus.jl_b200/csrc/residual.h) against the division, on the CPU: the header is
-compiled with the host compiler, whose division and fused multiply-add round as IEEE 754 says, as the device's do.
-Random operands over all exponents with the reciprocal up to three units off, as its callers' are: one unit from the
-division where the residual cannot underflow, seven below (the product alone); and zeros, infinities, NaN, subnormals and the largest numbers
-in every combination but a subnormal divisor, with the reciprocal the division gives: the same, but for a zero's sign."""
+"""The quotient and the root by residual correction (octopus.jl_b200/csrc/residual.h) against the division and the square
+root, on the CPU: the header is compiled with the host compiler, whose division, square root and fused multiply-add round
+as IEEE 754 says, as the device's do.  Random operands over all exponents with the reciprocal up to three units off, as
+its callers' are: one unit from the exact operation where the residual cannot underflow, seven below (the product alone);
+and zeros, infinities, NaN, subnormals and the largest numbers in every combination but a subnormal divisor, with the
+reciprocal the division gives: the same, but for a zero's sign."""
 import os
 import shutil
 import subprocess
@@ -45,7 +46,7 @@ int main() {
         std::uniform_real_distribution<double> u(-1.0, 1.0);
         const double x = std::ldexp(u(rng), (int)(rng() % 200) - 100), d = std::ldexp(u(rng), (int)(rng() % 200) - 100);
         if (d == 0.0) continue;
-        if (octo::quotient(x, d, 1.0 / d) != x / d) {
+        if (octo::quotient(x, d, 1.0 / d) != x / d || octo::quotient_in_range(x, d, 1.0 / d) != x / d) {
             std::printf("%a / %a: %a\n", x, d, octo::quotient(x, d, 1.0 / d));
             return 1;
         }
@@ -63,13 +64,27 @@ int main() {
                     return 1;
                 }
             }
+    for (int t = 0; t < 4000000; ++t) {
+        const double v = std::fabs(value(rng()));
+        if (std::fpclassify(v) != FP_NORMAL) continue;
+        const double want = std::sqrt(v);
+        double rs = 1.0 / want;
+        const int off = (int)(rng() % 7) - 3;
+        for (int k = 0; k < (off < 0 ? -off : off); ++k) rs = std::nextafter(rs, off < 0 ? -INFINITY : INFINITY);
+        const double got = octo::root(v, rs);
+        const int64_t away = bits(got) - bits(want), limit = v >= 0x1p-960 ? 1 : 7;
+        if (away > limit || away < -limit) {
+            std::printf("root of %a (%d off): %a, sqrt %a\n", v, off, got, want);
+            return 1;
+        }
+    }
     std::puts("ok");
     return 0;
 }
 """
 
 
-def test_quotient_against_the_division(tmp_path):
+def test_quotient_and_root_against_the_exact_operations(tmp_path):
     cxx = shutil.which("g++")
     if cxx is None:
         pytest.skip("no host C++ compiler")
