@@ -58,6 +58,27 @@ def test_kick_of_every_regime(aspect, n):
     assert np.max(np.abs(got[5] - p[5])) <= 2e-12 * np.max(np.abs(p[5])) + 1e-16
 
 
+@pytest.mark.parametrize("aspect", [1.0, 1.0 + 5e-4, 1.02, 11.0, 1.0 / 11.0, 150.0])
+def test_hessians_of_every_regime(aspect):
+    """A source whose momenta are correlated with its positions: the longitudinal kick then holds both Hessians."""
+    sy = 1e-5
+    e, p = _source(4001, aspect * sy, sy), _probes(aspect * sy, sy, 441)
+    e[1], e[3] = 3.0 * e[0], -2.0 * e[2]  # au = 2 cov(x, px) = 6 sigma_x^2, du = -4 sigma_y^2 at zero drift
+    lum, ref, got = _collide(e, p)
+    assert abs(lum / ref - 1.0) < 1e-12
+    # The momenta as in test_kick_of_every_regime, and with their error dK, 2 x 4.4e-16 x 2.51 / sqrt(q^2 - 1) over the
+    # short sigma (q the aspect ratio, at most 84 in its place near round): a Hessian is (x Kx + y Ky - 2 (1 - ..)) over the
+    # difference of the variances, so over some three sigma its error is 3 (q + 1) dK / (q^2 - 1) in units of 1 / short^2,
+    # and never less than a few roundings of its largest term; times a quarter of au, 6 q^2 / 4 long variances.
+    q = max(aspect, 1.0 / aspect)
+    amp = min(2.51 / np.sqrt(max(q * q - 1.0, 1e-9)), 84.0)
+    dk = 2 * 4.4e-16 * amp
+    dh = 3.0 * (q + 1.0) * dk / max(q * q - 1.0, 8.8e-4) + 1e-14 / (q * q)
+    bound = 2.0 * 1.5 * q * q * dh
+    assert np.max(np.abs(got[5] - p[5])) <= bound + 1e-14 * np.max(np.abs(p[5])), (np.max(np.abs(got[5] - p[5])), bound)
+    assert np.max(np.abs(p[5])) > 0.5  # the Hessian terms are there
+
+
 @pytest.mark.parametrize("aspect", [11.0, 1.0 / 11.0, 150.0])
 def test_particles_far_outside(aspect):
     """Coordinates whose square over the variance overflows: no density, and the kick of a distant charge."""
