@@ -28,6 +28,7 @@ constexpr int kMomentChunk = 8;         // rows of order >= 3 per generic pass (
 constexpr int kMomentPairs = 21;        // second-order rows: the products of deviations (i <= j)
 constexpr int kMomentsMax = 256;
 constexpr int kMomentSums1 = 6 + kMomentPairs + 1;  // k_moment_pass: deviations, their products, the live count
+constexpr int kMeanBlocks = 592, kMeanSums = 7;      // k_moment_means: partial-sum blocks; deviations, the live count
 
 // Rows of order >= 3 of one generic pass.
 struct MomentPowers {
@@ -222,6 +223,53 @@ __global__ void __launch_bounds__(kMomentThreads, 2) k_moment_pass(const __grid_
     block_sums<kMomentSums1>(s, red, partial);
 }
 
+// The pass of a row without second-order moments: the deviations alone.  Its pivot only has to lie within some sigma of
+// the mean, so each block takes it from the beam's first 32 particles (their mean where that is more than four of their
+// rms spreads from zero, else zero) and k_moment_pivot is not launched.  Bound by HBM; four blocks a
+// SM with one particle in flight a thread (two, or five and six blocks within fewer registers, measured no better).
+// 2.56M and 100,000 float64 particles, orders (1,): 36 and 13 us a row; 46 and 21 by k_moment_pass with its products.
+template <class R>
+__global__ void __launch_bounds__(kMomentThreads, 4) k_moment_means(const __grid_constant__ MomentBeam<R> B, double *pivots,
+                                                                    double *partial) {
+    pdl_wait();
+    pdl_release();
+    __shared__ double red[kMeanSums * kMomentWarps], pivot[6];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp < 6) {
+        double c[6], t[3] = {0.0, 0.0, 0.0};
+        if (lane < B.n) {
+            load6(c, B.c[0], B.c[1], B.c[2], B.c[3], B.c[4], B.c[5], lane);
+            const double v = (double)B.c[warp][lane];
+            if (isfinite(v) && (!B.mask || live6(c))) {
+                t[0] = v;
+                t[1] = v * v;
+                t[2] = 1.0;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
+        const double mean = t[0] / t[2];
+        if (lane == 0) {
+            pivot[warp] = isfinite(mean) && !(17.0 * mean * mean <= 16.0 * (t[1] / t[2])) ? mean : 0.0;
+            if (blockIdx.x == 0) pivots[warp] = pivot[warp];
+        }
+    }
+    __syncthreads();
+    double s[kMeanSums] = {};
+#pragma unroll 1
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < B.n; i += (long long)gridDim.x * blockDim.x) {
+        double c[6];
+        load6(c, B.c[0], B.c[1], B.c[2], B.c[3], B.c[4], B.c[5], i);
+        if (B.mask && !live6(c)) continue;
+#pragma unroll
+        for (int d = 0; d < 6; ++d) s[d] += c[d] - pivot[d];
+        s[6] += 1.0;
+    }
+    block_sums<kMeanSums>(s, red, partial);
+}
+
 // Fixed-order sum of partial[b * stride + k] over b < nb by one block of kMomentThreads threads: thread t
 // takes b = t, t + kMomentThreads, ... in order, then the block's fixed shuffle/warp tree.
 __device__ __forceinline__ double fold_partials(const double *partial, int nb, int stride, int k) {
@@ -242,7 +290,7 @@ __device__ __forceinline__ double fold_partials(const double *partial, int nb, i
 // block 0 also the live count means[6] and the row's turn; block 6 + k: requested pair k, NaN where a mean it
 // involves is not finite, as the deviations from such a mean are.  The four columns a pair takes are folded together.
 __global__ void __launch_bounds__(kMomentThreads) k_moment_finish(const double *pivots, const double *partial, int nb,
-                                                                  double turn, const __grid_constant__ MomentHead head,
+                                                                  int sums, double turn, const __grid_constant__ MomentHead head,
                                                                   const __grid_constant__ MomentPairRows Q,
                                                                   double *means, double *row) {
     pdl_wait();
@@ -257,11 +305,11 @@ __global__ void __launch_bounds__(kMomentThreads) k_moment_finish(const double *
         while (pair >= first + 6 - a) first += 6 - a++;
         b = a + pair - first;
     }
-    const int col[4] = {kMomentSums1 - 1, a, b, 6 + pair};
+    const int col[4] = {sums - 1, a, b, q >= 0 ? 6 + pair : a};
     double t[4] = {0.0, 0.0, 0.0, 0.0};
     for (int p = threadIdx.x; p < nb; p += kMomentThreads)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) t[k] += partial[(size_t)p * kMomentSums1 + col[k]];
+        for (int k = 0; k < 4; ++k) t[k] += partial[(size_t)p * sums + col[k]];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
 #pragma unroll

@@ -2810,7 +2810,7 @@ int32_t octo_beam_moments(octo_ctx *c, const octo_beam *beam, const int32_t *pow
     cudaStream_t st = (cudaStream_t)stream;
     try {
         CK(cudaSetDevice(c->device));
-        c->mom_partial.ensure((size_t)kMomentBlocks * kMomentSums1);
+        c->mom_partial.ensure((size_t)kMomentBlocks * kMomentSums1);  // more than kMeanBlocks * kMeanSums
         c->mom_means.ensure(24);
         const long long n = beam->n;
         const int mask = mask_lost != 0;
@@ -2820,12 +2820,16 @@ int32_t octo_beam_moments(octo_ctx *c, const octo_beam *beam, const int32_t *pow
             const double *means = c->mom_means.p;
             const MomentBeam<R> mb{{b[0], b[1], b[2], b[3], b[4], b[5]}, n, mask};
             double *pivots = c->mom_means.p + 16;
-            launch_pdl(k_moment_pivot<R>, 6, kPivotThreads, 0, st, mb, pivots);
-            launch_pdl(k_moment_pass<R>, kMomentBlocks, kMomentThreads, 0, st, mb, (const double *)pivots,
-                       c->mom_partial.p);
+            if (pairs.n) {
+                launch_pdl(k_moment_pivot<R>, 6, kPivotThreads, 0, st, mb, pivots);
+                launch_pdl(k_moment_pass<R>, kMomentBlocks, kMomentThreads, 0, st, mb, (const double *)pivots,
+                           c->mom_partial.p);
+            } else {
+                launch_pdl(k_moment_means<R>, kMeanBlocks, kMomentThreads, 0, st, mb, pivots, c->mom_partial.p);
+            }
             launch_pdl(k_moment_finish, 6 + pairs.n, kMomentThreads, 0, st, (const double *)pivots,
-                       (const double *)c->mom_partial.p, (int)kMomentBlocks, (double)turn, head, pairs, c->mom_means.p,
-                       row);
+                       (const double *)c->mom_partial.p, pairs.n ? kMomentBlocks : kMeanBlocks,
+                       pairs.n ? kMomentSums1 : kMeanSums, (double)turn, head, pairs, c->mom_means.p, row);
             for (size_t g0 = 0; g0 < general.size(); g0 += kMomentChunk) {
                 MomentPowers P{};
                 P.n = (int)std::min<size_t>(kMomentChunk, general.size() - g0);

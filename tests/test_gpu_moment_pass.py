@@ -79,7 +79,7 @@ def _live_row(c, dtype):
     c = c.astype(np.float32).astype(np.float64) if dtype == torch.float32 else c
     obs = ob.MomentObserver("b", orders=(1, 2), mask_lost=True)
     obs.observe(0, ob.Beam.from_numpy(c, ob.BeamParams(1.0, 1.0, 1.0, 1.0, 1.0), dtype=dtype))
-    return obs.rows()[0], c[:, np.isfinite(c).all(axis=0)].astype(np.longdouble)
+    return obs.rows()[0], np.ascontiguousarray(c[:, np.isfinite(c).all(axis=0)], dtype=np.longdouble)
 
 
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
@@ -108,3 +108,33 @@ def test_lost_particles_leave_the_pivot(case, far, dtype):
             own = 1e-32 * abs(mean[i] * mean[j])
             assert abs(row[k] - (d[i] * d[j]).mean()) <= 1e-13 * rms[i] * rms[j] + own + 1e-300, (i, j, row[k])
             k += 1
+
+
+@pytest.mark.parametrize("kind", ["plain", "sorted", "stray", "offset", "equal", "lost"])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 4097, 592 * 256 + 1, 400_003])
+def test_rows_without_second_moments(n, dtype, kind):
+    """Rows of order 1, and of 1 and 3, sum the deviations without their products, about a pivot of their own."""
+    import octo_b200 as ob
+    c = _beam("offset" if kind == "lost" else kind, n)
+    if kind == "lost":
+        c[:, 1::3] = 1e6
+        c[2, 1::3] = np.nan
+    if dtype == torch.float32:
+        c = c.astype(np.float32).astype(np.float64)
+    live = np.ascontiguousarray(c[:, np.isfinite(c).all(axis=0)], dtype=np.longdouble)  # rows of pairwise sums
+    mean = live.mean(axis=1)
+    d = live - mean[:, None]
+    rms = np.sqrt((d * d).mean(axis=1))
+    for orders in ((1,), (1, 3)):
+        obs = ob.MomentObserver("b", orders=orders, mask_lost=kind == "lost")
+        obs.observe(4, ob.Beam.from_numpy(c, ob.BeamParams(1.0, 1.0, 1.0, 1.0, 1.0), dtype=dtype))
+        row = dict(zip(obs.column_names, obs.rows()[0]))
+        got = np.array([row["m" + "0" * k + "1" + "0" * (5 - k)] for k in range(6)])
+        # the bounds of test_row_matches_extended_precision
+        np.testing.assert_array_less(np.abs(got - mean), 1e-13 * rms + 2.3e-16 * np.abs(mean) + 1e-300)
+        if 3 in orders:
+            for k in range(6):
+                third = (d[k] ** 3).mean()
+                assert abs(row["m" + "0" * k + "3" + "0" * (5 - k)] - third) <= 1e-12 * max(rms[k] ** 3, (abs(d[k]) ** 3).mean()) \
+                    + 1e-15 * abs(mean[k]) * rms[k] ** 2 + 1e-300
