@@ -173,8 +173,8 @@ struct Cnn {
     // which takes the parts of K on CTAs of their own, their fp32 sums added by the bias / ReLU / bf16 epilogue kernel.
     // skip != null: the layer's input is [nearest-upsampled in (cu channels), skip] (a decoder level), read
     // directly instead of a materialised concatenation.  pooled != null: the layer's input is the 2x2 average of in;
-    // a GEMM takes it from pooled, which this then fills.
-    void conv(int l, const bf16 *in, int B, bf16 *out_bf, float *out_f, cudaStream_t st, const bf16 *skip = nullptr,
+    // a GEMM takes it from pooled, which this then fills.  Returns the launches.
+    int conv(int l, const bf16 *in, int B, bf16 *out_bf, float *out_f, cudaStream_t st, const bf16 *skip = nullptr,
               int cu = 0, bf16 *pooled = nullptr) {
         const LayerSpec &L = kLayers[l];
         ConvArgs c{};
@@ -186,14 +186,14 @@ struct Cnn {
         c.error = err;
         const Parts parts = conv_parts(l, B);
         c.parts = parts.n; c.part_steps = parts.chunks * (kBK / 16);
-        if (launch_conv(c, B, st)) return;
+        if (launch_conv(c, B, st)) return 1;
         if (pooled) {
             pool(in, pooled, B, L.level - 1, L.cin, st);
             in = pooled;
         }
-        gemm_conv(l, in, B, out_bf, out_f, st, skip, cu);
+        return (pooled ? 1 : 0) + gemm_conv(l, in, B, out_bf, out_f, st, skip, cu);
     }
-    void gemm_conv(int l, const bf16 *in, int B, bf16 *out_bf, float *out_f, cudaStream_t st, const bf16 *skip, int cu) {
+    int gemm_conv(int l, const bf16 *in, int B, bf16 *out_bf, float *out_f, cudaStream_t st, const bf16 *skip, int cu) {
         const LayerSpec &L = kLayers[l];
         GemmArgs a{};
         a.M = (int)ml(L.level, B); a.N = L.cout; a.K = 9 * L.cin;
@@ -209,7 +209,7 @@ struct Cnn {
         const int used = parts.n;
         if (used == 1) {
             launch_gemm(a, 1, st);
-            return;
+            return 1;
         }
         a.k_per_split = parts.chunks * kBK;
         splitbuf.ensure((size_t)used * a.M * L.cout);
@@ -218,6 +218,7 @@ struct Cnn {
         launch_gemm(a, used, st);
         launch_pdl(k_umma_split_epilogue, ew_blocks((long long)a.M * L.cout), 256, 0, st, (const float *)splitbuf.p, used,
                    (long long)a.M, L.cout, (const float *)(master.p + boff[l]), L.relu, out_bf, (long long)L.cout);
+        return 2;
     }
 
     void pool(const bf16 *in, bf16 *o, int B, int level, int C, cudaStream_t st) {
@@ -230,41 +231,46 @@ struct Cnn {
     }
 
     // Forward pass of B inputs already in x0; the head's fp32 output lands in `out` ([M0][8]).  Inference
-    // (materialize = false) reads each decoder level's [upsampled, skip] input inside the GEMM; training keeps
-    // the concatenations, whose transposed im2col the weight gradients read.
-    void forward(int B, cudaStream_t st, bool materialize = true) {
-        if (weights_dirty) refresh_weights(st);
-        if (!materialize) {
-            conv(L_E1A, x0.p, B, a0.p, nullptr, st);
-            conv(L_E1B, a0.p, B, s1.p, nullptr, st);
-            conv(L_E2A, s1.p, B, a2.p, nullptr, st, nullptr, 0, p1.p);
-            conv(L_E2B, a2.p, B, s2.p, nullptr, st);
-            conv(L_E3A, s2.p, B, a4.p, nullptr, st, nullptr, 0, p2.p);
-            conv(L_E3B, a4.p, B, s3.p, nullptr, st);
-            conv(L_B, s3.p, B, b6.p, nullptr, st, nullptr, 0, p3.p);
-            conv(L_D3, b6.p, B, d7.p, nullptr, st, s3.p, 128);
-            conv(L_D2, d7.p, B, d8.p, nullptr, st, s2.p, 64);
-            conv(L_D1, d8.p, B, d9.p, nullptr, st, s1.p, 32);
-            conv(L_HEAD, d9.p, B, nullptr, out.p, st);
-            return;
+    // (materialize = false) reads each pooled input and each decoder level's [upsampled, skip] input inside the
+    // convolution; training keeps them, whose transposed im2col the weight gradients read.  Returns the launches.
+    int forward(int B, cudaStream_t st, bool materialize = true) {
+        int n = 0;
+        if (weights_dirty) {
+            refresh_weights(st);
+            n += kCnnLayers;
         }
-        conv(L_E1A, x0.p, B, a0.p, nullptr, st);
-        conv(L_E1B, a0.p, B, s1.p, nullptr, st);
+        if (!materialize) {
+            n += conv(L_E1A, x0.p, B, a0.p, nullptr, st);
+            n += conv(L_E1B, a0.p, B, s1.p, nullptr, st);
+            n += conv(L_E2A, s1.p, B, a2.p, nullptr, st, nullptr, 0, p1.p);
+            n += conv(L_E2B, a2.p, B, s2.p, nullptr, st);
+            n += conv(L_E3A, s2.p, B, a4.p, nullptr, st, nullptr, 0, p2.p);
+            n += conv(L_E3B, a4.p, B, s3.p, nullptr, st);
+            n += conv(L_B, s3.p, B, b6.p, nullptr, st, nullptr, 0, p3.p);
+            n += conv(L_D3, b6.p, B, d7.p, nullptr, st, s3.p, 128);
+            n += conv(L_D2, d7.p, B, d8.p, nullptr, st, s2.p, 64);
+            n += conv(L_D1, d8.p, B, d9.p, nullptr, st, s1.p, 32);
+            n += conv(L_HEAD, d9.p, B, nullptr, out.p, st);
+            return n;
+        }
+        n += conv(L_E1A, x0.p, B, a0.p, nullptr, st);
+        n += conv(L_E1B, a0.p, B, s1.p, nullptr, st);
         pool(s1.p, p1.p, B, 0, 32, st);
-        conv(L_E2A, p1.p, B, a2.p, nullptr, st);
-        conv(L_E2B, a2.p, B, s2.p, nullptr, st);
+        n += conv(L_E2A, p1.p, B, a2.p, nullptr, st);
+        n += conv(L_E2B, a2.p, B, s2.p, nullptr, st);
         pool(s2.p, p2.p, B, 1, 64, st);
-        conv(L_E3A, p2.p, B, a4.p, nullptr, st);
-        conv(L_E3B, a4.p, B, s3.p, nullptr, st);
+        n += conv(L_E3A, p2.p, B, a4.p, nullptr, st);
+        n += conv(L_E3B, a4.p, B, s3.p, nullptr, st);
         pool(s3.p, p3.p, B, 2, 128, st);
-        conv(L_B, p3.p, B, b6.p, nullptr, st);
+        n += conv(L_B, p3.p, B, b6.p, nullptr, st);
         upcat(b6.p, s3.p, u3.p, B, 2, 128, 128, st);
-        conv(L_D3, u3.p, B, d7.p, nullptr, st);
+        n += conv(L_D3, u3.p, B, d7.p, nullptr, st);
         upcat(d7.p, s2.p, u2.p, B, 1, 64, 64, st);
-        conv(L_D2, u2.p, B, d8.p, nullptr, st);
+        n += conv(L_D2, u2.p, B, d8.p, nullptr, st);
         upcat(d8.p, s1.p, u1.p, B, 0, 32, 32, st);
-        conv(L_D1, u1.p, B, d9.p, nullptr, st);
-        conv(L_HEAD, d9.p, B, nullptr, out.p, st);
+        n += conv(L_D1, u1.p, B, d9.p, nullptr, st);
+        n += conv(L_HEAD, d9.p, B, nullptr, out.p, st);
+        return n + 6;  // the pools and the concatenations
     }
 
     // out[(tap * C + c)][m] of an NHWC tensor (TAPS = 1: its transpose), 32 channels a block or 8

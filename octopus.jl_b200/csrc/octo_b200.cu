@@ -1595,8 +1595,7 @@ void CollideJob::run() {
                                              "plane count (" + std::to_string(F.np) + ")"};
             c->cnn_q.ensure((size_t)c->cnn->net.maxB);
             launch_pdl(k_cnn_prep, F.np, 256, 0, st, C, F.p0, c->cnn->net.x0.p, c->cnn_q.p);
-            c->cnn->net.forward(F.np, st, false);
-            launches += 1 + 17;
+            launches += 1 + c->cnn->net.forward(F.np, st, false);
         }
         if (c->cap_armed && !c->cap_taken) {
             for (int t = F.t0; t < F.t0 + F.nt; ++t) {

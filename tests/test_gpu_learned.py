@@ -106,3 +106,22 @@ def test_learned_form_field_error_against_bassetti_erskine(coarse):
             err = field_error(solver, aspect * sy, sy, dtype, 0, correction=(net, L.OUT_SCALE, 1e30, L.EDGE))
             assert err["rms"] < 0.01, (coarse, aspect, dtype, err)
     net.close()
+
+
+def test_reported_launches_count_the_network():
+    """A learned collide launches the input, the network's eleven layers and the correction beside each front."""
+    import torch
+    import octo_b200 as ob
+    from octo_b200 import learned as L
+    solver = L.coarse_solver("pic", 32, slicing=ob.LongitudinalSlicing(nslices=5, method="normal_quantile"))
+    net = L.FieldCorrectionNet(32, 32, max_batch=32)
+    e, p = _beams(ob, 20000, 10000, torch.float64)
+    counts = []
+    for form in (ob.Context(solver, 0, torch.float64), None):
+        form = form or L.LearnedForm(solver, solver, net, tolerance=1e9, dtype=torch.float64)
+        for _ in range(2):  # the first pass of a network also lays its weights out
+            form.collide(ob.Beam(e.coords.clone(), e.params), ob.Beam(p.coords.clone(), p.params), turn=1)
+            counts.append(getattr(form, "ctx", form).last_report.kernel_launches)
+    fronts = 9
+    assert counts[2] - counts[0] == fronts * (1 + 11 + 1) + 11
+    assert counts[3] - counts[1] == fronts * (1 + 11 + 1)
