@@ -1008,6 +1008,7 @@ struct CollideJob {
     int compute_lum;
     octo_collide_report *rep;
     cudaStream_t st;
+    int sharing = 1;  // collides enqueued side by side (a batch's count): block counts that fill the device take a share
     long long launches = 0;
     bool fp32 = false;
     size_t rsz = sizeof(double);
@@ -1479,7 +1480,8 @@ void CollideJob::run() {
         // blocks per slice of the bounds passes: 2048 particles each, fewer (down to one a thread) where that leaves
         // less than four blocks per SM -- the extrema do not depend on the split; the hybrid's moments and :sigma's
         // sums do, so theirs stays
-        const long long coarse = std::max<long long>(1, 2 * npf * ((F.maxsrc + 2047) / 2048)), want = 4LL * c->num_sms;
+        const long long sms = std::max(1, c->num_sms / sharing);  // this collide's own share of the device
+        const long long coarse = std::max<long long>(1, 2 * npf * ((F.maxsrc + 2047) / 2048)), want = 4LL * sms;
         const long long per = gaussian || c->dopt.grid_extent || coarse >= want ? 2048 : std::max<long long>(256, 2048 * coarse / want);
         const unsigned bps = (unsigned)std::max<long long>(1, std::min<long long>(kMaxBoundBlocks, (F.maxsrc + per - 1) / per));
         bool union_first = false;
@@ -1524,7 +1526,7 @@ void CollideJob::run() {
                 // uniform blocks per side: this stream runs beside the front's deposit and convolution and wants
                 // parallelism (blocks in proportion to each side's slice, sized to whole waves, measured slower)
                 // 32,768 particles each, fewer (down to 2,048) where the front would leave SMs without a block
-                const long long lper = std::max<long long>(2048, std::min<long long>(32768, 2 * F.nl * F.maxlum / c->num_sms));
+                const long long lper = std::max<long long>(2048, std::min<long long>(32768, 2 * F.nl * F.maxlum / sms));
                 unsigned bpp = (unsigned)std::max<long long>(1, std::min<long long>(8, (F.maxlum + lper - 1) / lper));
                 with_real(fp32, [&](auto r) {
                     launch_method(lmethod, [&](auto M) {
@@ -2635,7 +2637,7 @@ int32_t octo_pic_collide_batch(int32_t count, octo_ctx *const *ctxs, octo_beam *
         octo_collide_report *r = reports ? reports + k : nullptr;
         if (r) { std::memset(r, 0, sizeof(*r)); r->turn = turn; }
         jobs.push_back(CollideJob{ctxs[k], beam1[k], beam2[k], p1[k], p2[k], turn, compute_luminosity, r,
-                                  streams ? (cudaStream_t)streams[k] : (cudaStream_t)0});
+                                  streams ? (cudaStream_t)streams[k] : (cudaStream_t)0, count});
         if (luminosity) luminosity[k] = NAN;
         if (ctxs[k]->opt.nx == 0) rc[k] = fail(ctxs[k], OCTO_ERR_UNSUPPORTED, ctxs[k]->err.empty() ? "invalid context" : ctxs[k]->err);
     }
