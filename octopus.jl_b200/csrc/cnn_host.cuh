@@ -35,7 +35,7 @@ inline long long round8(long long v) { return (v + 7) / 8 * 8; }
 inline unsigned ew_blocks(long long n) { return (unsigned)std::max<long long>(1, std::min<long long>((n + 255) / 256, 148 * 16)); }
 
 struct Cnn {
-    int device = 0, H = 0, W = 0, maxB = 0;
+    int device = 0, sms = 148, H = 0, W = 0, maxB = 0;
     long long nparams = 0;
     long long woff[kCnnLayers] = {0}, boff[kCnnLayers] = {0};
     DevBuf<float> master, grad, adam_m, adam_v;
@@ -61,6 +61,7 @@ struct Cnn {
     void create(int dev, int h, int wd, int maxb, uint64_t seed) {
         device = dev; H = h; W = wd; maxB = maxb;
         CK(cudaSetDevice(device));
+        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
         long long off = 0;
         for (int l = 0; l < kCnnLayers; ++l) {
             woff[l] = off;
@@ -186,7 +187,7 @@ struct Cnn {
         c.error = err;
         const Parts parts = conv_parts(l, B);
         c.parts = parts.n; c.part_steps = parts.chunks * (kBK / 16);
-        if (launch_conv(c, B, st)) return 1;
+        if (launch_conv(c, B, sms, st)) return 1;
         if (pooled) {
             pool(in, pooled, B, L.level - 1, L.cin, st);
             in = pooled;
@@ -322,7 +323,7 @@ struct Cnn {
         c.out = fa.p;
         c.parts = 1; c.part_steps = 9 * (L.cout / 16);
         c.error = err;
-        if (launch_conv(c, B, st)) return;
+        if (launch_conv(c, B, sms, st)) return;
         GemmArgs a{};
         a.M = (int)ml(L.level, B); a.N = L.cin; a.K = 9 * L.cout;
         a.A = g.p; a.a_mode = 1; a.H = hl(L.level); a.W = wl(L.level); a.C = L.cout;

@@ -39,7 +39,7 @@ constexpr int kConvThreads = 256;
 struct ConvArgs {
     const bf16 *in, *skip;   // skip: null, or [b][H][W][C - Cu] beside the upsampled in [b][H/2][W/2][Cu]
     int Cu, pool;            // pool: in is [b][2H][2W][C]
-    int H, W, C;             // C = 8 or a multiple of 16; Cu a multiple of 8
+    int H, W, C;             // C = 8 or a multiple of 16 with C / 8 a divisor of the block; Cu a multiple of 8
     const bf16 *w;           // [N][3][3][C]
     int N;                   // output channels (row length of the output)
     const float *bias;       // null: none
@@ -66,8 +66,8 @@ inline size_t conv_smem(int C, int nb, int plane) {
 // channels, 12 x 12, 20 images) ran 240 CTAs in two waves, 31 us; now one band an image, 80 CTAs, 19 us.
 constexpr size_t kConvSmem = 226 * 1024;
 constexpr double kConvNone = 1e30;
-inline double conv_plan(ConvArgs &g, int B, int nb) {
-    if (g.C % 16 && g.C != 8) return kConvNone;
+inline double conv_plan(ConvArgs &g, int B, int nb, int sms) {
+    if ((g.C % 16 && g.C != 8) || kConvThreads % (g.C / 8)) return kConvNone;
     const int wp = g.W + 2, nblk = (g.N + nb - 1) / nb, steps = conv_chunks(g.C) / 2;
     double best = kConvNone;
     for (int R = 1; R <= g.H; ++R) {
@@ -80,7 +80,7 @@ inline double conv_plan(ConvArgs &g, int B, int nb) {
         while (cols < tiles * nb * g.parts) cols *= 2;
         const long long ctas = (long long)((g.H + R - 1) / R) * B * nblk;
         const int res = (int)std::min<long long>({(long long)(228 * 1024 / (smem + 2048)), 512 / cols, 8});
-        const double per_sm = (double)((ctas + 147) / 148), waves = (double)((ctas + 148LL * res - 1) / (148LL * res));
+        const double per_sm = (double)((ctas + sms - 1) / sms), waves = (double)((ctas + (long long)sms * res - 1) / ((long long)sms * res));
         const double cost = 4.0 * waves + per_sm * (smem * 8.3e-6 + 0.008 * tiles * steps * (nb / 16));
         if (cost < best) {
             best = cost;
@@ -144,14 +144,12 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3(const __grid_constant__ 
     // input rows y0 - 1 .. y0 + rows, zero outside the image
     {
         // One 16-byte chunk of a pixel a step: the chunks of a pixel lie side by side in memory, so neighbouring
-        // threads take them.  Where 256 is a multiple of c8 a thread keeps its chunk and walks the pixels by additions
+        // threads take them.  256 is a multiple of c8, so a thread keeps its chunk and walks the pixels by additions
         // alone (with a division or two a chunk this loop was the layer's longest part).
         const int Cs = g.C - g.Cu, pixels = (rows + 2) * wp;
-        const bool walk = kConvThreads % c8 == 0;
-        const int dp = walk ? kConvThreads / c8 : 1, dy = dp / wp, dx = dp - dy * wp;
-        int k = tid % c8, p = walk ? tid / c8 : 0, y = y0 - 1 + p / wp, x = p % wp - 1;
-        if (!walk && tid >= c8) p = pixels;  // c8 threads take every pixel (no network of this library's)
-        for (; p < pixels; p += dp) {
+        const int dp = kConvThreads / c8, dy = dp / wp, dx = dp - dy * wp;
+        const int k = tid % c8;
+        for (int p = tid / c8, y = y0 - 1 + p / wp, x = p % wp - 1; p < pixels; p += dp) {
             const int c = k * 8;
             const uint32_t dst = sA + (uint32_t)((k * g.plane + p) * 16);
             const bool in = y >= 0 && y < g.H && x >= 0 && x < g.W;

@@ -257,9 +257,9 @@ void launch_gemm(const GemmArgs &g, int splits, cudaStream_t st) {
 }
 
 // A 3x3 convolution of B images by bands (k_conv.cuh); false when no band of the image fits a CTA.
-bool launch_conv(ConvArgs g, int B, cudaStream_t st) {
+bool launch_conv(ConvArgs g, int B, int sms, cudaStream_t st) {
     ConvArgs wide = g;
-    const double narrow_cost = conv_plan(g, B, 16), wide_cost = g.N <= 16 ? kConvNone : conv_plan(wide, B, 32);
+    const double narrow_cost = conv_plan(g, B, 16, sms), wide_cost = g.N <= 16 ? kConvNone : conv_plan(wide, B, 32, sms);
     if (std::min(narrow_cost, wide_cost) == kConvNone) return false;
     const int nb = wide_cost <= narrow_cost ? 32 : 16;
     if (nb == 32) g = wide;

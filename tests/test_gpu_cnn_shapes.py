@@ -52,3 +52,9 @@ def test_forward_of_bands_that_fill_shared_memory(B, H, W):
     ref = co.Net(p.astype(np.float64), rounding=True).forward(xb.float().cpu().numpy().astype(np.float64))[..., :2]
     assert np.linalg.norm(out - ref) <= 1e-2 * np.linalg.norm(ref)  # the bound of test_gpu_cnn.py
     net.close()
+
+
+@pytest.mark.parametrize("W", [344, 1024, 2304])
+def test_gradients_where_no_band_fits(W):
+    """Wide images, whose forward layers and input gradients run as GEMMs: one, half of them, all."""
+    test_gradients_at_odd_sizes(1, 16, W, True)

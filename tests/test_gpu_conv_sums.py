@@ -102,3 +102,10 @@ def test_layers_in_parts(B, H, W, odd):
 
 def test_more_images_than_a_grid_axis_takes():
     _check(65537, 16, 16, False)
+
+
+@pytest.mark.parametrize("W", [344, 512, 1024, 2304])
+def test_images_too_wide_for_bands(W):
+    """From 344 columns on the widest decoder layer's band no longer fits shared memory and it runs as a GEMM, split over
+    K; at 1024 half of the layers do, at 2304 all of them, the pooled ones on a pooled copy of their input."""
+    _check(2, 16, W, True)
