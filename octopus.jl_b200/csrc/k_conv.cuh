@@ -61,9 +61,11 @@ inline size_t conv_smem(int C, int nb, int plane) {
 
 // Rows a band for B images at nb channels a CTA: the least of a launch's fixed latency per wave, the bytes each SM brings
 // in and the instructions it issues, over the bands that fit (TMEM, half of it for a sum in one part, and kConvSmem:
-// 227 KB less the 1 KB of this kernel itself).  Returns that cost (about a microsecond a unit), 1e30 when none fits (very
-// wide images: the im2col GEMM runs those).  While bands were held to 200 KB the widest decoder layer (256 to 64
-// channels, 12 x 12, 20 images) ran 240 CTAs in two waves, 31 us; now one band an image, 80 CTAs, 19 us.
+// 227 KB less the 1 KB of this kernel itself).  Returns that cost, in microseconds: the three weights are a least-squares
+// fit to the 33 launches of forward passes over 1, 20 and 64 images of 48 x 48 (5.4 to 34 us each, cold caches under ncu),
+// which it gives within 12 % rms; 1e30 when no band fits (very wide images: the im2col GEMM runs those).  While bands were
+// held to 200 KB the widest decoder layer (256 to 64 channels, 12 x 12, 20 images) ran 240 CTAs in two waves, 31 us; now
+// one band an image, 80 CTAs, 19 us.
 constexpr size_t kConvSmem = 226 * 1024;
 constexpr double kConvNone = 1e30;
 inline double conv_plan(ConvArgs &g, int B, int nb, int sms) {
@@ -81,7 +83,7 @@ inline double conv_plan(ConvArgs &g, int B, int nb, int sms) {
         const long long ctas = (long long)((g.H + R - 1) / R) * B * nblk;
         const int res = (int)std::min<long long>({(long long)(228 * 1024 / (smem + 2048)), 512 / cols, 8});
         const double per_sm = (double)((ctas + sms - 1) / sms), waves = (double)((ctas + (long long)sms * res - 1) / ((long long)sms * res));
-        const double cost = 4.0 * waves + per_sm * (smem * 8.3e-6 + 0.008 * tiles * steps * (nb / 16));
+        const double cost = 5.8 * waves + per_sm * (smem * 1.5e-5 + 0.026 * tiles * steps * (nb / 16));
         if (cost < best) {
             best = cost;
             g.R = R;
