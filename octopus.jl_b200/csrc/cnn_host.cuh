@@ -101,7 +101,11 @@ struct Cnn {
         b6.ensure(M3 * 128); u3.ensure(M2 * 256); d7.ensure(M2 * 64); u2.ensure(M1 * 128); d8.ensure(M1 * 32);
         u1.ensure(M0 * 64); d9.ensure(M0 * 32); out.ensure(M0 * 8);
         const long long ld0 = round8(M0);
-        g.ensure(M0 * 32); gt.ensure(32 * ld0 + 64); colt.ensure(576 * ld0 + 64);
+        g.ensure(M0 * 32); gt.ensure(32 * ld0 + 64);
+        long long taps = 0;  // the widest transposed im2col of wgrad
+        for (const LayerSpec &L : kLayers)
+            taps = std::max(taps, (column_shifts(L.level) ? 3 : 9) * L.cin * round8(ml(L.level, maxB)));
+        colt.ensure(taps + 64);
         fa.ensure(M0 * 64); dc.ensure(M0 * 8 + 64); ds1.ensure(M0 * 32); ds2.ensure(M1 * 64); ds3.ensure(M2 * 128);
         long long pmax = 0;
         for (int l = 0; l < kCnnLayers; ++l) {
@@ -285,15 +289,17 @@ struct Cnn {
                        M, hh, ww, C, ld);
     }
 
+    // Whether a level's weight-gradient GEMMs take their nine taps from three column shifts of the transposed input (a
+    // third of the writes, and reads that L2 holds): where 8 pixels lie in one row; else the whole transposed im2col.
+    bool column_shifts(int level) const { return wl(level) % 8 == 0; }
+
     // Weight and bias gradients of layer l from its input activation and the bf16 output gradient in g.
     void wgrad(int l, const bf16 *in, int B, cudaStream_t st) {
         const LayerSpec &L = kLayers[l];
         const long long M = ml(L.level, B), ld = round8(M);
         const int hh = hl(L.level), ww = wl(L.level);
         im2col_t<1>((const bf16 *)g.p, gt.p, M, hh, ww, L.cout, ld, st);
-        // where 8 pixels lie in one row the GEMM takes its nine taps from three column shifts (a third of the writes,
-        // and reads that L2 holds); else from the whole transposed im2col
-        const bool shifts = ww % 8 == 0;
+        const bool shifts = column_shifts(L.level);
         if (shifts) im2col_t<3>(in, colt.p, M, hh, ww, L.cin, ld, st);
         else im2col_t<9>(in, colt.p, M, hh, ww, L.cin, ld, st);
         const int splits = wgrad_splits(l, B);
