@@ -8,7 +8,7 @@
 // rounded once on store; all element arithmetic is FP64.
 //
 // A map alone is bound by HBM, the lines by FP64 issue: block-diagonal maps run their 18 operations of 66 (kPlanar),
-// divisors that are constant or shared are divided by once (quotient), and Box-Muller's angle takes sincospi.  Both
+// divisors that are constant or shared are divided by once (quotient, residual.h), and Box-Muller's angle takes sincospi.  Both
 // rings' lines of a production turn (2.56M + 1.024M particles, 21 elements, four launches): 371 -> 308 us.
 //
 // Per-element constants that the reference evaluates per particle but that depend only on parameters
@@ -281,7 +281,7 @@ __device__ __forceinline__ void rad_plane(double &q, double &p, const double *e,
     const double u2 = line_uniform(rng, k2, particle, turn, smix_tp);
     const double rr = sqrt(-2.0 * log(u1));
     double s, co;
-    sincospi(2.0 * u2, &s, &co);  // of 2 pi u2 unrounded: its reduction is exact and a few instructions
+    sincospi(2.0 * u2, &s, &co);  // of 2 pi u2 unrounded
     const double n1 = rr * co, n2 = rr * s;
     q += e[0] * n1;
     p += e[1] * n2 + e[2] * n1;

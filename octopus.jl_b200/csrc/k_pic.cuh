@@ -65,8 +65,8 @@ struct Collide {           // device pointers for one collide (passed by value)
 
 // ------------------------------------------------------------------ bounds
 // Running extrema, acc first.  A NaN v leaves acc, as fmin and fmax do, and is flagged separately; which zero of a
-// +-0 tie is kept changes no geometry.  A double's comparison and selection are three instructions where fmin's full
-// rules are about six (FP32 has the minimum in hardware).
+// +-0 tie is kept changes no geometry.  In float64 a comparison and a selection measured faster than fmin and fmax
+// (k_pair_bounds' figures below); float32 has no such difference.
 __device__ __forceinline__ double vmin(double acc, double v) { return v < acc ? v : acc; }
 __device__ __forceinline__ double vmax(double acc, double v) { return v > acc ? v : acc; }
 __device__ __forceinline__ float vmin(float acc, float v) { return fminf(acc, v); }
@@ -100,8 +100,8 @@ __device__ __forceinline__ unsigned long long shfl_max_u64(unsigned long long v)
 // (drifted to sL and sR, pic_cpu.jl:961-1003), field of the other (drifted to its collision
 // point, pic_cpu.jl:1005-1035) and luminosity source (drifted to sM, pic_cpu.jl:1279-1287).
 // Per-thread extrema (vmin, vmax) are encoded to ordered integers once per block for the atomics.  Bound by issue,
-// not HBM: the extrema of one particle are twelve comparisons, and fmin / fmax with a NaN test per drifted value took
-// three times the instructions (a hybrid turn of 1.28M + 0.512M particles, 15 slices: 7.25 -> 6.88 ms; the node boxes,
+// not HBM: the extrema of one particle are twelve comparisons; with fmin / fmax and a NaN test per drifted value it
+// took longer (a hybrid turn of 1.28M + 0.512M particles, 15 slices: 7.25 -> 6.88 ms; the node boxes,
 // which share the change, take 0.1 ms off the production turn of 6.31 ms).
 // grid: (blocks per side, 2 * pairs in front).
 template <class R>
