@@ -45,9 +45,9 @@ CONFIG = {
     "luminosity": "every turn", "precision": "fp64 plain form (int64 fixed-point charge grids)",
     "l2": "inputs larger than L2 (172 MB of particle coordinates per turn)",
 }
-# DRAM bytes (read + write) per field particle of one kick launch, from one `ncu --set full` capture of
-# the 15-pair front of this workload (276.9 MB for 3.584M field particles).
-KICK_TRAFFIC_BYTES_PER_PARTICLE = 77.3
+# DRAM bytes (read + write) per field particle of one kick launch, from one `ncu` capture of the 15-pair front of
+# this workload (274.8 MB for 3.584M field particles).
+KICK_TRAFFIC_BYTES_PER_PARTICLE = 76.7
 
 
 def _dist():

@@ -66,7 +66,7 @@ struct Collide {           // device pointers for one collide (passed by value)
 // ------------------------------------------------------------------ bounds
 // Running extrema, acc first.  A NaN v leaves acc, as fmin and fmax do, and is flagged separately; which zero of a
 // +-0 tie is kept changes no geometry.  In float64 a comparison and a selection measured faster than fmin and fmax
-// (k_pair_bounds' figures below); float32 has no such difference.
+// (k_pair_bounds' figures below); float32 keeps fminf and fmaxf.
 __device__ __forceinline__ double vmin(double acc, double v) { return v < acc ? v : acc; }
 __device__ __forceinline__ double vmax(double acc, double v) { return v > acc ? v : acc; }
 __device__ __forceinline__ float vmin(float acc, float v) { return fminf(acc, v); }
