@@ -160,7 +160,7 @@ struct Cnn {
 
     // Parts of K in which layer l's sums over a batch of B are added, in order, and the 64-wide chunks of each but the
     // last: where a GEMM's 128-row output tiles are too few to fill the GPU (the coarse levels), enough to fill it
-    // twice, no shorter than two chunks.
+    // twice, no shorter than two chunks.  148 SMs whatever the device has: the sums' rounding depends on the parts.
     struct Parts {
         int n, chunks;
     };
